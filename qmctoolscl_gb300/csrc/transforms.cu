@@ -22,9 +22,13 @@
 // and so on.  The FFT runs the low-bit pass first, the inverse the high-bit
 // pass first, matching the order of their stages.
 //
-// GB300 runs FP64 at about 1.25 TFLOP/s, so these kernels are FP64-bound;
-// they are the plain, reference-accurate path.  The tensor-core path
-// (tc_fft.cu) is the fast one.
+// GB300 runs FP64 at about 1.25 TFLOP/s, so these FP64 stages (ft_pass_kernel) are bound by the
+// FP64 unit.  From 2^9 values on the passes of fix_transform.cuh take their place: the same
+// transform with each tile in 64-bit block fixed point on the integer and IMAD pipes (errors
+// against long double: 0.3-0.9 of the FP64 stages' on normal, spiky, smooth and nearly
+// constant data, n = 2^9..2^18).  Device time, FP64 stages -> fixed point: FFT of
+// 32 x 2^20 4500 -> 1070 us, IFFT of 111 x 2^10 17.2 -> 16.6, WHT of 300 x 2^16 845 -> 144.
+// The tensor-core path (tc_fft.cu) is faster still at 1e-7.
 #include <cmath>
 
 #include "common.cuh"
@@ -37,14 +41,45 @@ constexpr u32 TILE_REAL = 8192;
 
 enum FtKind { FT_FFT = 0, FT_IFFT = 1, FT_FWHT = 2, FT_CONV = 3, FT_WCONV = 4 };
 
-__global__ void twiddle_kernel(u64 n, double sign, double *twr, double *twi)
+__device__ void fill_fix_entry(u32 t);
+
+// twiddles of an n-point transform, then (more = 4096 + 256) the tables of the fixed-point passes.
+// From n = 8 on a thread takes one angle of the first eighth turn and writes its eight mirror
+// images: the same bits (sincospi reduces to that eighth itself) for an eighth of the FP64 work,
+// n = 2^20: 73 -> 15 us.
+__global__ void twiddle_kernel(u64 n, double sign, double *twr, double *twi, u32 more)
 {
-    for (u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (u64)gridDim.x * blockDim.x) {
+    const u64 count = n >= 8 ? n / 8 + 1 : n;
+    for (u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x; t < count + more; t += (u64)gridDim.x * blockDim.x) {
+        if (t >= count) {
+            fill_fix_entry((u32)(t - count));
+            continue;
+        }
         double sn, cs;
         // the angle 2*pi*t/n as a multiple of pi is exact for n a power of two
         sincospi(__ddiv_rn(__ull2double_rn(2 * t), __ull2double_rn(n)), &sn, &cs);
-        twr[t] = cs;
-        twi[t] = sign * sn;
+        if (n < 8) {
+            twr[t] = cs;
+            twi[t] = sign * sn;
+            continue;
+        }
+        const u64 q = n / 4;
+        double c = cs, s = sn;  // of the angle t + k n / 4
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            twr[t + k * q] = c;
+            twi[t + k * q] = sign * s;
+            // the mirror image about the middle of the quarter: (k + 1) n / 4 - t
+            const double mc = k & 1 ? -cs : sn, ms = k & 1 ? sn : cs;
+            const u64 i = (k + 1) * q - t;
+            if (t > 0 && t < n / 8) {
+                twr[i] = k & 2 ? -mc : mc;
+                twi[i] = sign * (k & 2 ? -ms : ms);
+            }
+            const double nc = 0.0 - s;  // turn by a quarter (a zero stays +0)
+            s = c;
+            c = nc;
+        }
     }
 }
 
@@ -61,6 +96,10 @@ struct PassArgs {
     const double *lr, *li;
     u32 lam_all, divide;
     double lam_scale;
+    // the fixed-point passes: the write-back scale as 2^scale_exp (times sqrt(1/2)); conj: the
+    // inverse steps read the forward transform's table
+    int scale_exp;
+    bool scale_odd, conj;
 };
 
 // the imaginary part of a twiddle; conjugated when the inverse steps read the
@@ -73,7 +112,7 @@ __device__ __forceinline__ double tw_im(double v) { return CONJ ? -v : v; }
 // c0 .. c0+ct-1.
 template <int KIND, bool CONJ>
 __device__ __forceinline__ void ft_stages(const PassArgs &a, double *sr, double *si, u64 h, u64 c0, u32 ct,
-                                          u32 tile_elems)
+                                          u32 tile_elems, u32 nt)
 {
     const u32 nb = tile_elems / 2;
     const u32 nbits = a.k1 - a.k0;
@@ -90,7 +129,7 @@ __device__ __forceinline__ void ft_stages(const PassArgs &a, double *sr, double 
             // at bit 0 every twiddle is 1: the same step without the products (a separate loop,
             // so the FP64 multiplies are skipped rather than predicated off)
             if (KIND != FT_FWHT && bit == 0) {
-                for (u32 b = threadIdx.x; b < tile_elems / 4; b += FT_THREADS) {
+                for (u32 b = threadIdx.x; b < tile_elems / 4; b += nt) {
                     const u32 p = b / ct, cc = b % ct;
                     const u32 e0 = (p << 2) * ct + cc, e1 = e0 + S, e2 = e1 + S, e3 = e2 + S;
                     const double x0r = sr[e0], x0i = si[e0], x1r = sr[e1], x1i = si[e1];
@@ -122,7 +161,7 @@ __device__ __forceinline__ void ft_stages(const PassArgs &a, double *sr, double 
                 __syncthreads();
                 continue;
             }
-            for (u32 b = threadIdx.x; b < tile_elems / 4; b += FT_THREADS) {
+            for (u32 b = threadIdx.x; b < tile_elems / 4; b += nt) {
                 const u32 p = b / ct, cc = b % ct;
                 const u32 q0 = ((p >> hb) << (hb + 2)) | (p & ((1u << hb) - 1));
                 const u32 e0 = q0 * ct + cc, e1 = e0 + S, e2 = e1 + S, e3 = e2 + S;
@@ -182,7 +221,7 @@ __device__ __forceinline__ void ft_stages(const PassArgs &a, double *sr, double 
             continue;
         }
         const u32 half = 1u << hb;
-        for (u32 b = threadIdx.x; b < nb; b += FT_THREADS) {
+        for (u32 b = threadIdx.x; b < nb; b += nt) {
             const u32 p = b / ct, cc = b % ct;
             const u32 q1 = ((p >> hb) << (hb + 1)) | (p & (half - 1));
             const u32 e1 = q1 * ct + cc, e2 = e1 + half * ct;
@@ -212,6 +251,45 @@ __device__ __forceinline__ void ft_stages(const PassArgs &a, double *sr, double 
             }
         }
         __syncthreads();
+    }
+}
+
+// The stages of one pass on a tile in shared memory and, for the fused forms, the pointwise step
+// between the forward and the inverse ones: y <- y * lam * f or y / lam * f (f = scale / n: the
+// orthonormal factors of both transforms), lam n values shared by the vectors or one per element.
+template <int KIND, bool CONJ>
+__device__ __forceinline__ void ft_tile(const PassArgs &a, double *sr, double *si, u64 base, u64 h, u64 c0, u32 ct,
+                                        u32 tile_elems, u32 nt)
+{
+    constexpr bool REAL = KIND == FT_FWHT || KIND == FT_WCONV;
+    const u64 n = 1ull << a.m;
+    if constexpr (KIND == FT_CONV || KIND == FT_WCONV) {
+        ft_stages<KIND == FT_CONV ? (int)FT_FFT : (int)FT_FWHT, false>(a, sr, si, h, c0, ct, tile_elems, nt);
+        const double f = a.lam_scale;
+        for (u32 e = threadIdx.x; e < tile_elems; e += nt) {
+            const u32 q = e / ct, cc = e % ct;
+            const u64 gi = base + ((u64)q << a.k0) + cc;
+            const u64 li = a.lam_all ? gi : (gi & (n - 1));
+            const double lr = a.lr[li];
+            if (REAL) {
+                sr[e] = a.divide ? sr[e] * f / lr : sr[e] * lr * f;
+            } else {
+                const double lm = a.li[li], yr = sr[e] * f, yi = si[e] * f;
+                if (a.divide) {
+                    const double den = fma(lr, lr, lm * lm);
+                    sr[e] = fma(yr, lr, yi * lm) / den;
+                    si[e] = fma(yi, lr, -yr * lm) / den;
+                } else {
+                    sr[e] = fma(yr, lr, -yi * lm);
+                    si[e] = fma(yr, lm, yi * lr);
+                }
+            }
+        }
+        __syncthreads();
+        ft_stages<KIND == FT_CONV ? (int)FT_IFFT : (int)FT_FWHT, KIND == FT_CONV>(a, sr, si, h, c0, ct, tile_elems,
+                                                                                 nt);
+    } else {
+        ft_stages<KIND, CONJ>(a, sr, si, h, c0, ct, tile_elems, nt);
     }
 }
 
@@ -246,36 +324,7 @@ __global__ void __launch_bounds__(FT_THREADS) ft_pass_kernel(PassArgs a)
             if (!REAL) si[e] = a.xi[gi];
         }
         __syncthreads();
-        if constexpr (KIND == FT_CONV || KIND == FT_WCONV) {
-            ft_stages<KIND == FT_CONV ? (int)FT_FFT : (int)FT_FWHT, false>(a, sr, si, h, c0, ct, tile_elems);
-            // y <- y * lam * f or y / lam * f (f = scale / n: the orthonormal factors of both
-            // transforms), lam n values shared by the vectors or one per element
-            const double f = a.lam_scale;
-            for (u32 e = threadIdx.x; e < tile_elems; e += FT_THREADS) {
-                const u32 q = e / ct, cc = e % ct;
-                const u64 gi = base + ((u64)q << a.k0) + cc;
-                const u64 li = a.lam_all ? gi : (gi & (n - 1));
-                const double lr = a.lr[li];
-                if (REAL) {
-                    sr[e] = a.divide ? sr[e] * f / lr : sr[e] * lr * f;
-                } else {
-                    const double lm = a.li[li], yr = sr[e] * f, yi = si[e] * f;
-                    if (a.divide) {
-                        const double den = fma(lr, lr, lm * lm);
-                        sr[e] = fma(yr, lr, yi * lm) / den;
-                        si[e] = fma(yi, lr, -yr * lm) / den;
-                    } else {
-                        sr[e] = fma(yr, lr, -yi * lm);
-                        si[e] = fma(yr, lm, yi * lr);
-                    }
-                }
-            }
-            __syncthreads();
-            ft_stages<KIND == FT_CONV ? (int)FT_IFFT : (int)FT_FWHT, KIND == FT_CONV>(a, sr, si, h, c0, ct,
-                                                                                    tile_elems);
-        } else {
-            ft_stages<KIND, CONJ>(a, sr, si, h, c0, ct, tile_elems);
-        }
+        ft_tile<KIND, CONJ>(a, sr, si, base, h, c0, ct, tile_elems, FT_THREADS);
         const double sc = a.scale;
         for (u32 e = threadIdx.x; e < tile_elems; e += FT_THREADS) {
             const u32 q = e / ct, cc = e % ct;
@@ -286,6 +335,39 @@ __global__ void __launch_bounds__(FT_THREADS) ft_pass_kernel(PassArgs a)
         __syncthreads();
     }
 }
+
+// One tile of a fixed-point pass in FP64 (tiles that hold inf, nan, zeros only or values near the
+// ends of the exponent range): starts from and ends with the data in global memory, and with
+// a barrier.
+template <int KIND>
+__device__ __noinline__ void fp64_tile(const PassArgs &a, double *sm, u64 base, u64 h, u64 c0, u32 ct, u32 tile_elems)
+{
+    constexpr bool REAL = KIND == FT_FWHT || KIND == FT_WCONV;
+    double *sr = sm, *si = sm + tile_elems;
+    const u32 nt = blockDim.x;
+    for (u32 e = threadIdx.x; e < tile_elems; e += nt) {
+        const u64 gi = base + ((u64)(e / ct) << a.k0) + e % ct;
+        sr[e] = a.xr[gi];
+        if (!REAL) si[e] = a.xi[gi];
+    }
+    __syncthreads();
+    if (KIND == FT_IFFT && a.conj)
+        ft_tile<KIND, true>(a, sr, si, base, h, c0, ct, tile_elems, nt);
+    else
+        ft_tile<KIND, false>(a, sr, si, base, h, c0, ct, tile_elems, nt);
+    for (u32 e = threadIdx.x; e < tile_elems; e += nt) {
+        const u64 gi = base + ((u64)(e / ct) << a.k0) + e % ct;
+        a.xr[gi] = sr[e] * a.scale;
+        if (!REAL) a.xi[gi] = si[e] * a.scale;
+    }
+    __syncthreads();
+}
+
+}  // namespace
+
+#include "fix_transform.cuh"
+
+namespace {
 
 struct Pass {
     u32 k0, k1, ct;
@@ -332,6 +414,93 @@ int launch_pass(int kind, bool conj, const PassArgs &a, unsigned grid, size_t sm
     }
 }
 
+// ---- the fixed-point passes
+
+// Few complex transforms of 2^9 are latency-bound, and the FP64 stages on 256 threads each
+// answer sooner than one warp does (64 vectors: 12.7 us against
+// 14.4; 300: 16.6 against 14.4; from 2^10 on fixed point wins from one vector: 15.6 against 17.9).
+bool use_fixed(bool real, u32 m, u64 nvec)
+{
+    return m > (u32)FIX_MIN_BITS || (m == (u32)FIX_MIN_BITS && (real || nvec >= (u64)qmcgb::sm_count()));
+}
+
+// Bits of the low pass of an m-bit transform: what is left above it is a multiple of four.
+u32 fix_low_bits(u32 m) { return m <= 12 ? m : 9 + (m - 9) % 4; }
+
+// Passes, low bits first: the low pass, then eight bits at a time, four in the last one where
+// eight do not remain.
+int plan_fix_passes(u32 m, Pass *out)
+{
+    int np = 0;
+    u32 k0 = fix_low_bits(m);
+    out[np++] = Pass{0, k0, 1};
+    while (k0 < m) {
+        const u32 s = m - k0 >= 8 ? 8 : 4;
+        out[np++] = Pass{k0, k0 + s, 4096u >> s};
+        k0 += s;
+    }
+    return np;
+}
+
+template <class K>
+int launch_fix(K kernel, const PassArgs &a, u64 tiles, unsigned threads, unsigned resident, size_t smem,
+               cudaStream_t s, const char *what)
+{
+    if (int rc = qmcgb::raise_smem_limit((const void *)kernel, smem, what)) return rc;
+    kernel<<<qmcgb::grid_for(tiles, 1, (unsigned)qmcgb::sm_count() * resident), threads, smem, s>>>(a);
+    return qmcgb::launch_status(what);
+}
+
+template <int KIND, int P>
+int launch_fix_low(const PassArgs &a, cudaStream_t s, const char *what)
+{
+    const u64 tiles = a.nvec << (a.m - P);
+    const size_t words = slots(1u << P);
+    if constexpr (KIND == FT_FWHT || KIND == FT_WCONV)
+        return launch_fix(fix_low_wht_kernel<KIND, P>, a, tiles, 1u << (P - 4), P == 12 ? 4 : (P == 11 ? 8 : (P == 10 ? 16 : 32)),
+                          words * 8, s, what);
+    else
+        return launch_fix(fix_low_kernel<KIND, P>, a, tiles, 1u << (P - 4), P == 12 ? 2 : (P == 11 ? 4 : (P == 10 ? 8 : 16)),
+                          words * 16, s, what);
+}
+
+template <int KIND, bool CONJ>
+int launch_fix_pass(const PassArgs &a, cudaStream_t s, const char *what)
+{
+    if (a.k0 == 0) {
+        switch (a.k1) {
+        case 9: return launch_fix_low<KIND, 9>(a, s, what);
+        case 10: return launch_fix_low<KIND, 10>(a, s, what);
+        case 11: return launch_fix_low<KIND, 11>(a, s, what);
+        default: return launch_fix_low<KIND, 12>(a, s, what);
+        }
+    }
+    const u64 tiles = (a.nvec << (a.m - a.k1)) * ((1ull << a.k0) / a.ct);
+    const size_t words = slots(4096);
+    const bool wide = a.k1 - a.k0 == 8;
+    if constexpr (KIND == FT_FWHT || KIND == FT_WCONV)
+        return wide ? launch_fix(fix_high_wht_kernel<KIND, 8>, a, tiles, 256, 4, words * 8, s, what)
+                    : launch_fix(fix_high_wht_kernel<KIND, 4>, a, tiles, 256, 4, words * 8, s, what);
+    else
+        return wide ? launch_fix(fix_high_kernel<KIND, CONJ, 8>, a, tiles, 256, 2, words * 16, s, what)
+                    : launch_fix(fix_high_kernel<KIND, CONJ, 4>, a, tiles, 256, 2, words * 16, s, what);
+}
+
+// one pass, in fixed point from 2^FIX_MIN_BITS values on
+int launch_any(int kind, bool conj, bool fixed, PassArgs a, unsigned grid, size_t smem, cudaStream_t s,
+               const char *what)
+{
+    if (!fixed) return launch_pass(kind, conj, a, grid, smem, s, what);
+    a.conj = conj;
+    switch (kind) {
+    case FT_FFT: return launch_fix_pass<FT_FFT, false>(a, s, what);
+    case FT_IFFT: return conj ? launch_fix_pass<FT_IFFT, true>(a, s, what) : launch_fix_pass<FT_IFFT, false>(a, s, what);
+    case FT_FWHT: return launch_fix_pass<FT_FWHT, false>(a, s, what);
+    case FT_CONV: return launch_fix_pass<FT_CONV, false>(a, s, what);
+    default: return launch_fix_pass<FT_WCONV, false>(a, s, what);
+    }
+}
+
 int run_transform(int kind, u64 d1, u64 d2, u64 n_half, double *twr, double *twi, double *xr, double *xi,
                   cudaStream_t s, const char *what)
 {
@@ -342,17 +511,18 @@ int run_transform(int kind, u64 d1, u64 d2, u64 n_half, double *twr, double *twi
     const u64 n = 2 * n_half;
     u32 m = 0;
     while ((1ull << m) < n) m++;
+    const bool fixed = use_fixed(kind == FT_FWHT || kind == FT_WCONV, m, nvec);
     if (kind != FT_FWHT) {
         QMC_REQUIRE(twr && twi, "%s: null twiddle pointer", what);
-        twiddle_kernel<<<qmcgb::grid_for(n, 256, (unsigned)qmcgb::sm_count() * 8), 256, 0, s>>>(
-            n, kind == FT_FFT ? -1.0 : 1.0, twr, twi);
+        twiddle_kernel<<<qmcgb::grid_for(n / 8 + 1 + (fixed ? 4096 + 256 : 8), 256, (unsigned)qmcgb::sm_count() * 8), 256, 0, s>>>(
+            n, kind == FT_FFT ? -1.0 : 1.0, twr, twi, fixed ? 4096 + 256 : 0);
         if (int rc = qmcgb::launch_status(what)) return rc;
     }
     if (nvec == 0) return QMC_OK;
     QMC_REQUIRE(xr && (kind == FT_FWHT || xi), "%s: null data pointer", what);
     const u32 tile = kind == FT_FWHT ? TILE_REAL : TILE_COMPLEX;
     Pass passes[16];
-    const int np = plan_passes(m, tile, passes);
+    const int np = fixed ? plan_fix_passes(m, passes) : plan_passes(m, tile, passes);
     // orthonormal scaling 2^(-m/2), applied once by the last pass
     const double scale = (m % 2 == 0) ? ldexp(1.0, -(int)(m / 2)) : ldexp(1.0, -(int)(m / 2)) * 0.70710678118654752440;
     for (int pi = 0; pi < np; pi++) {
@@ -368,11 +538,13 @@ int run_transform(int kind, u64 d1, u64 d2, u64 n_half, double *twr, double *twi
         a.twr = twr;
         a.twi = twi;
         a.scale = (pi == np - 1) ? scale : 1.0;
+        a.scale_exp = (pi == np - 1) ? -(int)(m / 2) : 0;
+        a.scale_odd = (pi == np - 1) && m % 2;
         const u32 elems = (1u << (p.k1 - p.k0)) * p.ct;
         const size_t smem = (size_t)elems * sizeof(double) * (kind == FT_FWHT ? 1 : 2);
         const u64 tiles = nvec * (n >> p.k1) * ((1ull << p.k0) / p.ct);
         const unsigned grid = qmcgb::grid_for(tiles, 1, (unsigned)qmcgb::sm_count() * 8);
-        if (int rc = launch_pass(kind, false, a, grid, smem, s, what)) return rc;
+        if (int rc = launch_any(kind, false, fixed, a, grid, smem, s, what)) return rc;
     }
     return QMC_OK;
 }
@@ -395,16 +567,18 @@ int run_fused(int kind, u64 d1, u64 d2, u64 n_half, double *twr, double *twi, co
     const u64 n = 2 * n_half;
     u32 m = 0;
     while ((1ull << m) < n) m++;
+    const bool fixed = use_fixed(kind == FT_FWHT || kind == FT_WCONV, m, nvec);
     if (!real) {
         QMC_REQUIRE(twr && twi, "%s: null twiddle pointer", what);
-        twiddle_kernel<<<qmcgb::grid_for(n, 256, (unsigned)qmcgb::sm_count() * 8), 256, 0, s>>>(n, -1.0, twr, twi);
+        twiddle_kernel<<<qmcgb::grid_for(n / 8 + 1 + (fixed ? 4096 + 256 : 8), 256, (unsigned)qmcgb::sm_count() * 8), 256, 0, s>>>(
+            n, -1.0, twr, twi, fixed ? 4096 + 256 : 0);
         if (int rc = qmcgb::launch_status(what)) return rc;
     }
     if (nvec == 0) return QMC_OK;
     QMC_REQUIRE(xr && lr && (real || (xi && li)), "%s: null data or lam pointer", what);
     const u32 tile = real ? TILE_REAL : TILE_COMPLEX;
     Pass passes[16];
-    const int np = plan_passes(m, tile, passes);
+    const int np = fixed ? plan_fix_passes(m, passes) : plan_passes(m, tile, passes);
     // launch order: forward passes 0 .. np-2, the fused pass np-1, inverse passes np-2 .. 0
     for (int li_ = 0; li_ < 2 * np - 1; li_++) {
         const int pi = li_ < np ? li_ : 2 * np - 2 - li_;
@@ -427,11 +601,20 @@ int run_fused(int kind, u64 d1, u64 d2, u64 n_half, double *twr, double *twi, co
         a.lam_all = (u32)lam_all;
         a.divide = divide ? 1u : 0u;
         a.lam_scale = scale / (double)n;
+        if (li_ == np - 1 && fixed) {  // a factor that is a power of two goes into the exponent
+            int ex = 0;
+            const double f = frexp(a.lam_scale, &ex);
+            if (f == 0.5 && ex > -900 && ex < 900) {
+                a.lam_scale = 1.0;
+                a.scale_exp = ex - 1;
+                a.scale = ldexp(1.0, ex - 1);
+            }
+        }
         const u32 elems = (1u << (p.k1 - p.k0)) * p.ct;
         const size_t smem = (size_t)elems * sizeof(double) * (real ? 1 : 2);
         const u64 tiles = nvec * (n >> p.k1) * ((1ull << p.k0) / p.ct);
         const unsigned grid = qmcgb::grid_for(tiles, 1, (unsigned)qmcgb::sm_count() * 8);
-        if (int rc = launch_pass(k, k == FT_IFFT, a, grid, smem, s, what)) return rc;
+        if (int rc = launch_any(k, k == FT_IFFT, fixed, a, grid, smem, s, what)) return rc;
     }
     return QMC_OK;
 }

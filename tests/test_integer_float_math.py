@@ -8,7 +8,9 @@ the host with g++ and checked against the host's IEEE arithmetic:
 * fpconv.cuh -- FP64 <-> FP32 conversions with round to nearest even
   (tensor-core transforms);
 * qrng_step.cuh -- one Horner step of halton_qrng, RN(RN(v + c) / b), over
-  random operands, ties and whole 32-step chains.
+  random operands, ties and whole 32-step chains;
+* fix64.cuh -- the block fixed-point arithmetic of the FP64 transforms, against
+  128-bit and long double arithmetic.
 """
 import os
 import shutil
@@ -61,5 +63,17 @@ def qrng_step_checker(tmp_path_factory):
 @pytest.mark.parametrize("seed", [1, 2])
 def test_qrng_step_matches_ieee(qrng_step_checker, seed):
     out = subprocess.run([qrng_step_checker, "3000000", str(seed)], capture_output=True, text=True, timeout=120)
+    assert out.returncode == 0, out.stdout + out.stderr
+    assert out.stdout.startswith("ok")
+
+
+@pytest.fixture(scope="module")
+def fix64_checker(tmp_path_factory):
+    return _compile(tmp_path_factory, "fix64_check.cpp")
+
+
+@pytest.mark.parametrize("seed", [1, 2])
+def test_block_fixed_point(fix64_checker, seed):
+    out = subprocess.run([fix64_checker, "200000", str(seed)], capture_output=True, text=True, timeout=120)
     assert out.returncode == 0, out.stdout + out.stderr
     assert out.stdout.startswith("ok")
