@@ -46,7 +46,11 @@
 // four digits is below half an ulp of v the lane stops.  The tile of doubles
 // is staged in shared memory and stored as contiguous rows.  The grid holds
 // exactly the CTAs resident at once, striding over the equal-cost tiles.
+// Plans of 24 million coordinates and more whose tables fit shared memory generate with
+// halton_rows_kernel (halton_rows.cuh) instead: first 100 primes, r=32, n=2^18, 20.3 -> 8.0 ms,
+// issue-bound (66 % of the issue slots, ALU 52 %, FP64 34 %) where this kernel waits for the FP64 unit.
 #include <algorithm>
+#include <cmath>
 #include <vector>
 
 #include "common.cuh"
@@ -73,6 +77,10 @@ struct HDim {
     u32 tpad;      // tmax rounded up to a multiple of HT_GROUP: term rows past tmax hold +0
     u64 fd_M;      // direct-remainder constant for b (any 32-bit x)
     u64 fdK_M;     // the same for b^K
+    // generation from shared-memory tables (halton_rows.cuh)
+    u32 t1, rows;  // FP64 rows at the front, rows that can change a sum of at least 2^-10
+    u32 K2, bK2;   // low digits of its index split, b^K2
+    u64 fdK2_M;
     u64 c_off;     // offset of this dimension's (mmax x tmax) block inside a randomisation's C block
     u64 y_off;     // offset of its (tpad x b) term rows inside a randomisation's Y block
     u64 s_off;     // offset of its tpad digits inside the request's tail blocks
@@ -95,6 +103,8 @@ struct HReq {
     double *x;
 };
 
+struct HGroup;
+
 struct HPlanDev {
     u64 nreq, total_c, rows, titems, ntiles, ndims;
     const HReq *req;
@@ -105,6 +115,10 @@ struct HPlanDev {
     const u32 *tail;     // largest biased exponent among the terms of digits t.. of (l, j)
     const u16 *order;    // per request, its dimension ids (request-relative) grouped by warp
     const u32 *wstart;   // per request, HT_WARPS + 1 offsets into its order
+    const HGroup *groups;
+    u32 ngroups;
+    const u32 *Cn, *mul;  // matrices divided by their lowest digit's row, and those divisors (numbered like tail)
+    const u32 *info;      // per (request, l, j): the sections of its rows
     unsigned *err;
 };
 
@@ -146,6 +160,8 @@ __device__ __forceinline__ u32 dim_mod(const HDim &D, u32 x)
 {
     return D.wide ? hmod(D.fd_M, D.b, x) : nmod(D.m32, D.b, x);
 }
+
+__device__ __forceinline__ u32 hr_term_flags(u64 y, u64 dig, u64 b);
 
 // ---------------------------------------------------------------- prep
 
@@ -214,7 +230,7 @@ __global__ void halton_recip_kernel(HPlanDev P, u64 *recip)
 // (64-bit wrapping add), then (double)digit * recip_t as
 // gdn_integer_to_float.c:36-37.  Lane 0 records the row's largest exponent in
 // the tail table (whose words are numbered exactly like the rows).
-__global__ void halton_terms_kernel(HPlanDev P, const PrepDim *pd, u64 *Y, u32 *tail)
+__global__ void halton_terms_kernel(HPlanDev P, const PrepDim *pd, u64 *Y, u32 *tail, u32 *flags)
 {
     const u32 lane = threadIdx.x % 32;
     const u64 wstride = (u64)gridDim.x * (blockDim.x / 32);
@@ -229,21 +245,27 @@ __global__ void halton_terms_kernel(HPlanDev P, const PrepDim *pd, u64 *Y, u32 *
         u64 *yrow = Y + R.y_base + l * R.y_per_l + D.y_off + t * D.b;
         if (t >= D.tmax) {  // padding row: +0 terms, no tail
             for (u32 g = lane; g < D.b; g += 32) yrow[g] = 0;
-            if (lane == 0) tail[row] = 0;
+            if (lane == 0) tail[row] = flags[row] = 0;
             continue;
         }
         const double rc = as_double(P.recip[D.r_off + t]);
         const u64 sh = R.has_shift ? Q.shifts[l * D.tmax + t] : 0;
         u64 mx = 0;
+        u32 fl = 0;
         for (u32 g = lane; g < D.b; g += 32) {
             const u64 pv = R.has_perm ? Q.perms[(l * D.tmax + t) * D.b + g] : g;
             const u64 dig = R.has_shift ? (pv + sh) % D.b : pv;
             const u64 y = dig ? as_bits(__dmul_rn(rc, __ull2double_rn(dig))) : 0;
             yrow[g] = y;
             mx = max(mx, y);  // non-negative doubles order like their bits
+            fl |= hr_term_flags(y, dig, D.b);
         }
+        fl = __reduce_or_sync(0xffffffffu, fl);
         for (int o = 16; o; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        if (lane == 0) tail[row] = (u32)(mx >> 52);
+        if (lane == 0) {
+            tail[row] = (u32)(mx >> 52);
+            flags[row] = fl;
+        }
     }
 }
 
@@ -464,6 +486,12 @@ __global__ void __launch_bounds__(HT_THREADS, 3) halton_gen_kernel(HPlanDev P, H
     }
 }
 
+}  // namespace
+
+#include "halton_rows.cuh"
+
+namespace {
+
 u64 ceil_digits(u64 n_last, u64 b)
 {
     u64 k = 0;
@@ -502,6 +530,10 @@ struct qmc_halton_plan {
     std::vector<PrepDim> prep;
     void *d_req = nullptr, *d_dims = nullptr, *d_C = nullptr, *d_Y = nullptr, *d_recip = nullptr, *d_tail = nullptr;
     void *d_order = nullptr, *d_wstart = nullptr, *d_prep = nullptr;
+    void *d_groups = nullptr, *d_Cn = nullptr, *d_mul = nullptr, *d_flags = nullptr, *d_info = nullptr;
+    u64 items = 0;       // CTAs of halton_rows_kernel; 0: some table does not fit
+    u32 rows_threads = 0;
+    size_t rows_smem = 0;
     size_t smem = 0;
     u32 ppl = 1;
     bool mixed = false;  // some dimensions add in integer arithmetic
@@ -520,6 +552,17 @@ void drop_graph(qmc_halton_plan *p)
     p->graph = nullptr;
 }
 
+// generation from shared-memory tables, unless one does not fit or some adds are to be integer ones
+// of the warp kernel
+bool use_rows(const qmc_halton_plan *p) { return p->items && !p->mixed; }
+
+int tail_launch(qmc_halton_plan *p, cudaStream_t st)
+{
+    const unsigned cap = (unsigned)qmcgb::sm_count() * 16;
+    halton_tail_kernel<<<qmcgb::grid_for(p->P.titems, 128, cap), 128, 0, st>>>(p->P, (u32 *)p->d_tail);
+    return qmcgb::launch_status("halton_tail_kernel");
+}
+
 int prepare_launch(qmc_halton_plan *p, cudaStream_t st)
 {
     const unsigned cap = (unsigned)qmcgb::sm_count() * 16;
@@ -529,10 +572,18 @@ int prepare_launch(qmc_halton_plan *p, cudaStream_t st)
     halton_recip_kernel<<<qmcgb::grid_for(p->P.ndims, 128, 1024), 128, 0, st>>>(p->P, (u64 *)p->d_recip);
     if (int rc = qmcgb::launch_status("halton_recip_kernel")) return rc;
     halton_terms_kernel<<<qmcgb::grid_for(p->P.rows * 32, 256, cap), 256, 0, st>>>(p->P, (const PrepDim *)p->d_prep,
-                                                                                  (u64 *)p->d_Y, (u32 *)p->d_tail);
+                                                                                  (u64 *)p->d_Y, (u32 *)p->d_tail,
+                                                                                  (u32 *)p->d_flags);
     if (int rc = qmcgb::launch_status("halton_terms_kernel")) return rc;
-    halton_tail_kernel<<<qmcgb::grid_for(p->P.titems, 128, cap), 128, 0, st>>>(p->P, (u32 *)p->d_tail);
-    return qmcgb::launch_status("halton_tail_kernel");
+    if (p->items) {
+        halton_norm_kernel<<<qmcgb::grid_for(p->P.rows, 128, cap), 128, 0, st>>>(p->P, (const u32 *)p->d_C,
+                                                                                (u32 *)p->d_Cn, (u32 *)p->d_mul);
+        if (int rc = qmcgb::launch_status("halton_norm_kernel")) return rc;
+        halton_info_kernel<<<qmcgb::grid_for(p->P.titems, 64, cap), 64, 0, st>>>(
+            p->P, (const u32 *)p->d_flags, (const u32 *)p->d_Cn, (u32 *)p->d_info);
+        if (int rc = qmcgb::launch_status("halton_info_kernel")) return rc;
+    }
+    return use_rows(p) ? QMC_OK : tail_launch(p, st);
 }
 
 // Every tile costs the same, and the CTAs stride over the tiles: a grid of exactly the CTAs
@@ -551,6 +602,10 @@ unsigned resident_grid(const qmc_halton_plan *p)
 
 int run_launch(qmc_halton_plan *p, cudaStream_t st)
 {
+    if (use_rows(p)) {
+        halton_rows_kernel<<<(unsigned)p->items, p->rows_threads, p->rows_smem, st>>>(p->P);
+        return qmcgb::launch_status("halton_rows_kernel");
+    }
     const HReq &R1 = p->hreq[0];
     const bool one = p->hreq.size() == 1, mixed = p->mixed;
 #define HT_LAUNCH(PPL_, ONE_, MIXED_)                                                             \
@@ -571,6 +626,75 @@ int run_launch(qmc_halton_plan *p, cudaStream_t st)
     }
 #undef HT_LAUNCH
     return qmcgb::launch_status("halton_gen_kernel");
+}
+
+// The groups of dimensions, CTAs and shared memory of halton_rows_kernel; leaves items 0 where
+// one dimension's tables do not fit or the work is too small for them.
+void plan_rows(qmc_halton_plan *p, std::vector<HGroup> &groups)
+{
+    const u64 sms = (u64)qmcgb::sm_count();
+    auto up = [](size_t v) { return (v + 15) & ~(size_t)15; };
+    const u32 nt = HR_THREADS, max_per = 16;
+    size_t smem = 0;
+    double work = 0, coords = 0;
+    std::vector<double> cost;
+    for (size_t q = 0; q < p->hreq.size(); q++) {
+        const HReq &R = p->hreq[q];
+        for (u64 j = 0; j < R.d;) {
+            HGroup G{};
+            G.req = (u32)q;
+            G.j0 = (u32)j;
+            size_t used = 0;
+            double c = 0;
+            while (j < R.d && G.nd < HR_DIMS && (G.nd == 0 || j % HR_DIMS)) {
+                const HDim &h = p->hd[R.dim0 + j];
+                const size_t pitch = 2 * (h.tmax | 1u), hs = up(((32 * max_per - 1) / h.bK2 + 2) * pitch);
+                const size_t T = up((size_t)h.tmax * h.b * 8), L = up(h.bK2 * pitch), H = hs * (nt / 32),
+                             C = up((size_t)h.mmax * h.tmax * 4);
+                if (used + T + L + H + C > HR_MAX_SMEM) break;
+                G.t_off[G.nd] = (u32)used;
+                G.l_off[G.nd] = (u32)(used + T);
+                G.h_off[G.nd] = (u32)(used + T + L);
+                G.c_off[G.nd] = (u32)(used + T + L + H);
+                G.h_size[G.nd] = (u32)hs;
+                used += T + L + H + C;
+                c += h.rows + 6.0;  // a step of a dimension: its rows, and about six rows' worth around them
+                G.nd++;
+                j++;
+            }
+            if (!G.nd) return;
+            smem = std::max(smem, used);
+            groups.push_back(G);
+            cost.push_back(c);
+            work += c * (double)R.r * (double)((R.n + nt - 1) / nt);
+            coords += (double)(R.r * R.n) * G.nd;
+        }
+    }
+    // The tables of a CTA cost about as much as two of its steps: it keeps them for up to 16 while
+    // there are a dozen CTAs of equal work per SM, heaviest (smallest bases) first.  Plans below
+    // HR_MIN_COORDS coordinates, or with fewer than HR_MIN_POINTS points per randomisation on
+    // average, finish sooner on the warp kernel, which has no tables to set up.
+    if (coords < HR_MIN_COORDS) return;
+    const double target = work / (12.0 * (double)sms);
+    u64 item0 = 0, randomisations = 0;
+    double points = 0;
+    for (const HReq &R : p->hreq) {
+        points += (double)R.r * (double)R.n;
+        randomisations += R.r;
+    }
+    if (points < HR_MIN_POINTS * (double)randomisations) return;
+    for (size_t g = 0; g < groups.size(); g++) {
+        HGroup &G = groups[g];
+        const HReq &R = p->hreq[G.req];
+        G.span = nt * std::max<u64>(HR_PTS, std::min<u64>(max_per, (u64)(target / cost[g])));
+        G.splits = (u32)((R.n + G.span - 1) / G.span);
+        G.item0 = item0;
+        item0 += R.r * G.splits;
+    }
+    if (item0 > 0x7FFFFFFFull) return;
+    p->items = item0;
+    p->rows_threads = nt;
+    p->rows_smem = smem;
 }
 
 template <u32 PPL>
@@ -663,6 +787,22 @@ int qmc_halton_batch_create(const qmc_halton_request *reqs, int nreq, qmc_halton
             h.fd_M = fastdiv32_make(h.b).M;
             h.fdK_M = fastdiv32_make(h.bK).M;
             h.tpad = (h.tmax + HT_GROUP - 1) / HT_GROUP * HT_GROUP;
+            // rows until b^t1 >= 2^16; rows whose terms (below b^-t) can reach half a last place of a
+            // sum of 2^-10 or more: 2^-63
+            const double bits = std::log2((double)h.b);
+            h.t1 = 1;
+            for (u64 v = h.b; v < (1ull << HR_HEAD_BITS) && h.t1 < h.tmax; v *= h.b) h.t1++;
+            h.rows = std::min<u32>(h.tmax, (u32)std::ceil((double)(54 + HR_TINY) / bits + 1e-9));
+            h.rows = std::max(h.rows, h.t1);
+            // low digits: one from b = 32 on, else as many as make a hundred values, so that a step's
+            // points share few values of the rest
+            h.K2 = 1;
+            h.bK2 = h.b;
+            while (h.b < 32 && h.bK2 < 100) {
+                h.bK2 *= h.b;
+                h.K2++;
+            }
+            h.fdK2_M = fastdiv32_make(h.bK2).M;
             h.c_off = c_off;
             h.y_off = y_off;
             h.s_off = s_off;
@@ -715,6 +855,8 @@ int qmc_halton_batch_create(const qmc_halton_request *reqs, int nreq, qmc_halton
         p->hreq.push_back(R);
     }
     p->mixed = assign_adds(p->hd, 1.0);
+    std::vector<HGroup> groups;
+    plan_rows(p, groups);
     const u64 ndims = p->hd.size();
     p->P.nreq = (u64)nreq;
     p->P.total_c = c_base;
@@ -739,6 +881,15 @@ int qmc_halton_batch_create(const qmc_halton_request *reqs, int nreq, qmc_halton
     alloc(&p->d_order, order.size() * sizeof(u16));
     alloc(&p->d_wstart, wstart.size() * sizeof(u32));
     alloc(&p->d_prep, ndims * sizeof(PrepDim));
+    alloc(&p->d_flags, t_base * sizeof(u32));
+    if (p->items) {
+        alloc(&p->d_groups, groups.size() * sizeof(HGroup));
+        alloc(&p->d_Cn, c_base * sizeof(u32));
+        alloc(&p->d_mul, t_base * sizeof(u32));
+        alloc(&p->d_info, tl_base * sizeof(u32));
+        put(p->d_groups, groups.data(), groups.size() * sizeof(HGroup));
+        if (!rc) rc = qmcgb::raise_smem_limit((const void *)halton_rows_kernel, p->rows_smem, "halton_rows_kernel smem");
+    }
     put(p->d_req, p->hreq.data(), nreq * sizeof(HReq));
     put(p->d_dims, p->hd.data(), ndims * sizeof(HDim));
     put(p->d_order, order.data(), order.size() * sizeof(u16));
@@ -754,6 +905,11 @@ int qmc_halton_batch_create(const qmc_halton_request *reqs, int nreq, qmc_halton
     p->P.tail = (const u32 *)p->d_tail;
     p->P.order = (const u16 *)p->d_order;
     p->P.wstart = (const u32 *)p->d_wstart;
+    p->P.groups = (const HGroup *)p->d_groups;
+    p->P.ngroups = (u32)groups.size();
+    p->P.Cn = (const u32 *)p->d_Cn;
+    p->P.mul = (const u32 *)p->d_mul;
+    p->P.info = (const u32 *)p->d_info;
     if (rc) {
         qmc_halton_plan_destroy(p);
         return rc;
@@ -818,15 +974,22 @@ int qmc_halton_plan_set_fp64_share(qmc_halton_plan *p, double share)
     if (int rc = qmcgb::cuda_status(cudaDeviceSynchronize(), "synchronise before rewriting the descriptors"))
         return rc;
     drop_graph(p);
-    return qmcgb::cuda_status(cudaMemcpy(p->d_dims, p->hd.data(), p->hd.size() * sizeof(HDim), cudaMemcpyHostToDevice),
-                              "copy");
+    if (int rc = qmcgb::cuda_status(
+            cudaMemcpy(p->d_dims, p->hd.data(), p->hd.size() * sizeof(HDim), cudaMemcpyHostToDevice), "copy"))
+        return rc;
+    if (!p->prepared || use_rows(p)) return QMC_OK;
+    // the warp kernel's stop table (a preparation for the other kernel left it out; a maximum over
+    // suffixes is its own maximum, so a second pass changes nothing)
+    if (int rc = tail_launch(p, nullptr)) return rc;
+    return qmcgb::cuda_status(cudaDeviceSynchronize(), "halton_tail_kernel");
 }
 
 int qmc_halton_plan_destroy(qmc_halton_plan *p)
 {
     if (!p) return QMC_OK;
     drop_graph(p);
-    for (void *q : {p->d_req, p->d_dims, p->d_C, p->d_Y, p->d_recip, p->d_tail, p->d_order, p->d_wstart, p->d_prep})
+    for (void *q : {p->d_req, p->d_dims, p->d_C, p->d_Y, p->d_recip, p->d_tail, p->d_order, p->d_wstart, p->d_prep,
+                    p->d_groups, p->d_Cn, p->d_mul, p->d_flags, p->d_info})
         if (q) cudaFree(q);
     delete p;
     return QMC_OK;
