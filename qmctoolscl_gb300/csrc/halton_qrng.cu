@@ -7,28 +7,35 @@
 // Horner's rule from digit 31 down, every add and divide rounded
 // (halton_qrng.c:133-140).  res is d x n, dimension-major.
 //
-// Bit for bit with less work: the digits at and above the index's digit
-// count m are zero, so the Horner steps over them are the same for every
-// point with m digits.  Each CTA owns one dimension and computes, once, the
-// prefix P[m] after the steps k = 31 .. m (P[0] is the reference's point 0);
-// a point then needs only its own m steps, each the reference's rounded add
-// and divide.  Three warps in four take them in integer arithmetic
-// (qrng_step.cuh), the fourth on the FP64 unit as the reference's own two
-// operations: on GB300 an FP64 divide is a sequence of several operations on a
-// narrow pipe, so neither kind of unit alone keeps up, and the two run side by
-// side (n = 2^20, d = 100: 2.82 ms with integer steps only, 2.51 ms with a
-// quarter of the warps on FP64; a third, a fifth, a sixth, or the FP64 warps
-// spread over the SM's sub-partitions, measured slower).  The digits come from
-// the top down by divisions by b^k (32-bit multiply-high, exact).
+// Bit for bit with less work.  The value after the steps k = 31 .. k0 depends on i / b^k0 alone, so
+// consecutive points share it: a CTA takes a dimension and 4096 consecutive points, computes the
+// values of the top level (the first k0 with at most 256 of them) each by its own chain, then
+// every level below from the one above with one step per value, and the points with one step
+// each: b / (b - 1) steps a point instead of its digit count.  Steps above an index's digits
+// add the digit shifts only and are the same for every point (P[m]).
+//
+// A step RN(RN(v + c) / b) takes four FP64 operations (qrng_step_fp64), or integer arithmetic
+// (qrng_step.cuh); of the last level, the one with all the points, every warp takes QRNG_INT_WARPS of
+// eight rounds in the integer form, so that the narrow FP64 unit and the integer pipes both work
+// (FP64 70 %, ALU 55 % busy: what bounds it, with the barriers between the levels).
+// n = 2^20, d = 100: 2.51 ms with the whole chains (a quarter of them by FP64 divides), 0.69 ms now.
+#include <algorithm>
+
 #include "common.cuh"
 #include "qrng_step.cuh"
 
 namespace {
 
-// the step with the FP64 operations, out of line, for what qstep::step leaves out
-__device__ __noinline__ u64 qrng_step_hw(u64 v, u32 c, double bd)
+// RN(RN(v + c) / b) for 0 <= v < 1 (v = 0 or above 2^-400) and integers 0 <= c < b < 2^12, rb = RN(1/b).
+// The division is one residual correction of a product by the rounded reciprocal (Markstein, IBM J. R&D
+// 1990).  Exact here: q0 = RN(x rb) is within 1.5 units of its last place of x/b, so x - q0 b is b times
+// that, a small integer multiple of a power of two, and the first fma has no error; q0 + r rb differs
+// from x/b by at most 2^-52 of a last place, while x/b lies at least 1/(2b) > 2^-13 of one from
+// every midpoint (it is never on one), so the second fma rounds as x/b itself.
+__device__ __forceinline__ double qrng_step_fp64(double v, double c, double b, double rb)
 {
-    return (u64)__double_as_longlong(__ddiv_rn(__dadd_rn(__longlong_as_double((long long)v), (double)c), bd));
+    const double x = __dadd_rn(v, c), q0 = __dmul_rn(x, rb);
+    return fma(fma(-q0, b, x), rb, q0);
 }
 
 constexpr int QRNG_DIMS = 360;
@@ -83,72 +90,102 @@ __constant__ int c_qrng_mult[QRNG_DIMS] = {
 };
 
 constexpr u32 QRNG_THREADS = 256;
+constexpr u32 QRNG_CHUNK = 4096;      // points of a step of a CTA (2048: 713 us, 1024: 810, against 689)
+constexpr u32 QRNG_MAX_B = 2424;
+constexpr u32 QRNG_INT_WARPS = 4;     // 0: 980 us, 2: 812, 3: 734, 4: 712, 5: 803 (n = 2^20, d = 100)
 
-// eight CTAs per SM (32 registers): each point's digit steps are one dependent chain, so
-// occupancy beats the few spilled registers (2, 3, 4, 6 CTAs per SM measured slower)
-__global__ void __launch_bounds__(QRNG_THREADS, 8) halton_qrng_kernel(int n, int n0, int generalized, double *res,
+struct QrngTables {
+    double level[2][QRNG_CHUNK / 2 + 2];  // the values of a level: odd levels in [1]
+    double c0[QRNG_MAX_B];                // the last step's addend by digit
+    double P[33];                         // prefix after the steps k = 31 .. m with digits 0
+    u32 s[32];                            // digit shifts
+};
+
+__global__ void __launch_bounds__(QRNG_THREADS, 4) halton_qrng_kernel(int n, int n0, int generalized, double *res,
                                                                    const double *randu, const int *dvec,
                                                                    unsigned *err)
 {
-    __shared__ double P[33];          // Horner prefix after the steps k = 31 .. m
-    __shared__ u32 s[32];             // digit shifts
-    __shared__ FastDiv32 pw[33];      // division by b^k, k < kmax
-    __shared__ u64 pwv[33];           // b^k (capped above 2^32)
-    __shared__ int b_s, f_s, ok_s;
-    const int j = blockIdx.y;
-    if (threadIdx.x == 0) {
-        const int idx = dvec[j];
-        ok_s = idx >= 0 && idx < QRNG_DIMS;
-        if (!ok_s) atomicOr(err, 1u);  // halton_qrng.c:70 would read outside its tables
-        b_s = ok_s ? c_qrng_prime[idx] : 2;
-        f_s = ok_s ? (generalized ? c_qrng_mult[idx] : 1) : 1;
+    extern __shared__ __align__(16) unsigned char sm[];
+    QrngTables &S = *(QrngTables *)sm;
+    const u32 tid = threadIdx.x;
+    const int j = blockIdx.y, idx = dvec[j];
+    if (idx < 0 || idx >= QRNG_DIMS) {  // halton_qrng.c:70 would read outside its tables
+        if (tid == 0) atomicOr(err, 1u);
+        return;
     }
+    const u32 b = (u32)c_qrng_prime[idx], f = generalized ? (u32)c_qrng_mult[idx] : 1u;
+    const double bd = (double)b, rb = __ddiv_rn(1.0, bd);
+    const FastDiv32 fb = fastdiv32_make(b);
+    const qstep::Div qd = qstep::make_div(b);
+    // halton_qrng.c:73: (int)(base * u), then stored as unsigned
+    if (tid < 32) S.s[tid] = (u32)__double2int_rz(__dmul_rn(bd, randu[(u64)j * 32 + tid]));
     __syncthreads();
-    if (!ok_s) return;
-    const int b = b_s;
-    const double bd = (double)b;
-    if (threadIdx.x < 32) {
-        // halton_qrng.c:73: (int)(base * u), then stored as unsigned
-        s[threadIdx.x] = (u32)__double2int_rz(__dmul_rn(bd, randu[(u64)j * 32 + threadIdx.x]));
-    }
-    if (threadIdx.x == 32) {
-        u64 v = 1;
-        for (int k = 0; k < 33; k++) {
-            pwv[k] = v;
-            pw[k] = fastdiv32_make((u32)(v >= 2 && v < (1ull << 32) ? v : 2u));  // k = 0 divides by 1 (unused)
-            v = v < (1ull << 32) ? v * (u64)b : v;
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {  // halton_qrng.c:74-78: u += s_k; u /= base, k = 31 .. 0
+    if (tid == 0) {  // halton_qrng.c:74-78: u += s_k; u /= base, k = 31 .. 0
         double u = 0.0;
-        P[32] = u;
+        S.P[32] = u;
         for (int k = 31; k >= 0; k--) {
-            u = __ddiv_rn(__dadd_rn(u, (double)s[k]), bd);
-            P[k] = u;
+            u = __ddiv_rn(__dadd_rn(u, (double)S.s[k]), bd);
+            S.P[k] = u;
         }
     }
+    // halton_qrng.c:135: the digit's addend
+    auto addend = [&](u32 digit, u32 k) { return fd_mod(fb, f * digit + S.s[k]); };
+    for (u32 g = tid; g < b; g += QRNG_THREADS) S.c0[g] = (double)addend(g, 0);
     __syncthreads();
-    const FastDiv32 fb = fastdiv32_make((u32)b);
-    const qstep::Div qd = qstep::make_div((u32)b);
-    const u32 f = (u32)f_s;
     double *out = res + (u64)j * (u64)n;
-    for (u64 q = (u64)blockIdx.x * QRNG_THREADS + threadIdx.x; q < (u64)n; q += (u64)gridDim.x * QRNG_THREADS) {
-        const u32 t = (u32)(int)((long long)n0 + (long long)q);  // halton_qrng.c:110: tmp = i
-        const bool fp64 = ((q >> 5) & 3u) == 0;                   // the warp's steps on the FP64 unit
-        int m = 0;  // base-b digit count of t (at most 32)
-        while (m < 32 && pwv[m + 1] <= (u64)t && pwv[m + 1] < (1ull << 32)) m++;
-        if (t) m++;
-        u64 v = (u64)__double_as_longlong(P[m]);
-        for (int k = m - 1; k >= 0; k--) {
-            const u32 top = k ? fd_div(pw[k], t) : t;       // t / b^k
-            const u32 dig = top - fd_div(fb, top) * (u32)b;  // its lowest digit: digit k of t
-            const u32 c = fd_mod(fb, f * dig + s[k]);       // halton_qrng.c:135
-            u64 o;                                          // halton_qrng.c:135-136: v = RN(RN(v + c) / b)
-            if (fp64 || !qstep::step(v, c, qd, o)) o = qrng_step_hw(v, c, bd);
-            v = o;
+    const u64 per = ((u64)n + gridDim.x - 1) / gridDim.x, q_end = min((u64)n, (blockIdx.x + 1) * per);
+    for (u64 q = blockIdx.x * per; q < q_end;) {
+        const u32 t0 = (u32)(int)((long long)n0 + (long long)q);  // halton_qrng.c:110: tmp = i
+        const u32 cnt = (u32)min(min(q_end - q, (u64)QRNG_CHUNK), (1ull << 32) - t0);  // a negative n0 wraps to 0
+        const u32 t1 = t0 + (cnt - 1);
+        // the top level
+        u32 K = 1, first = fd_div(fb, t0), last = fd_div(fb, t1);
+        while (last - first >= QRNG_THREADS) {
+            K++;
+            first = fd_div(fb, first);
+            last = fd_div(fb, last);
         }
-        out[q] = __longlong_as_double((long long)v);
+        if (tid <= last - first) {
+            u32 dig[32], m = K;
+            for (u32 h = first + tid; h; m++) {
+                const u32 up = fd_div(fb, h);
+                dig[m & 31u] = h - up * b;
+                h = up;
+            }
+            double v = S.P[m];
+            while (m-- > K) v = qrng_step_fp64(v, (double)addend(dig[m & 31u], m), bd, rb);
+            S.level[K & 1][tid] = v;
+        }
+        // the levels below it
+        for (u32 k = K - 1; k >= 1; k--) {
+            __syncthreads();
+            const u32 parent0 = first;
+            u32 lo = t0, hi = t1;
+            for (u32 i = 0; i < k; i++) {
+                lo = fd_div(fb, lo);
+                hi = fd_div(fb, hi);
+            }
+            for (u32 e = tid; e <= hi - lo; e += QRNG_THREADS) {
+                const u32 h = lo + e, up = fd_div(fb, h);
+                S.level[k & 1][e] =
+                    qrng_step_fp64(S.level[(k + 1) & 1][up - parent0], (double)addend(h - up * b, k), bd, rb);
+            }
+            first = lo;
+        }
+        __syncthreads();
+        // the points
+        for (u32 e = tid; e < cnt; e += QRNG_THREADS) {
+            const u32 t = t0 + e, up = fd_div(fb, t), digit = t - up * b;
+            const bool integer = ((e / QRNG_THREADS * 3 + tid / 32) & 7u) < QRNG_INT_WARPS;
+            const double v = S.level[1][up - first], c = S.c0[digit];
+            u64 o;
+            if (integer && qstep::step(as_bits(v), addend(digit, 0), qd, o))
+                out[q + e] = as_double(o);
+            else
+                out[q + e] = qrng_step_fp64(v, c, bd, rb);
+        }
+        __syncthreads();
+        q += cnt;
     }
 }
 
@@ -167,16 +204,16 @@ int qmc_halton_qrng(int n, int d, int n0, int generalized, double *res, const do
     QMC_REQUIRE(res && randu_d_32 && dvec, "halton_qrng: null array pointer");
     unsigned *err = qmcgb::device_error_ptr();
     QMC_REQUIRE(err, "device error word unavailable");
-    // about four waves of CTAs (eight per SM) over all dimensions, at least 64 per dimension:
-    // every CTA builds its dimension's tables first (a serial chain of FP64 divides), so
-    // fewer, longer CTAs cost less than one per few points (153 per dimension at d = 100
-    // measured 3 % slower than 64)
-    unsigned per_dim = (unsigned)(qmcgb::sm_count() * 8 * 4 / d);
-    if (per_dim < 64) per_dim = 64;
-    if (per_dim > (unsigned)qmcgb::sm_count() * 8) per_dim = (unsigned)qmcgb::sm_count() * 8;
-    const unsigned gx = qmcgb::grid_for((u64)n, QRNG_THREADS, per_dim);
-    halton_qrng_kernel<<<dim3(gx, (unsigned)d, 1), QRNG_THREADS, 0, QMC_STREAM(s)>>>(n, n0, generalized, res,
-                                                                                       randu_d_32, dvec, err);
+    // about eight waves of CTAs (four per SM) over all dimensions; a CTA builds its dimension's tables
+    // first, so it takes at least 1024 points (what is left of a chunk costs as much as the whole)
+    const u64 waves = (u64)qmcgb::sm_count() * 4 * 8;
+    u64 per_dim = std::max<u64>(1, waves / (u64)d);
+    per_dim = std::max<u64>(std::min<u64>(per_dim, ((u64)n + QRNG_CHUNK - 1) / QRNG_CHUNK),
+                            std::min<u64>(((u64)n + 1023) / 1024, (u64)qmcgb::sm_count() * 4 / (u64)d));
+    const unsigned gx = (unsigned)std::max<u64>(1, per_dim);
+    if (int rc = qmcgb::raise_smem_limit((const void *)halton_qrng_kernel, sizeof(QrngTables), "halton_qrng")) return rc;
+    halton_qrng_kernel<<<dim3(gx, (unsigned)d, 1), QRNG_THREADS, sizeof(QrngTables), QMC_STREAM(s)>>>(
+        n, n0, generalized, res, randu_d_32, dvec, err);
     return qmcgb::launch_status("halton_qrng");
 }
 
