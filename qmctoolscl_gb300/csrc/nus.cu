@@ -25,8 +25,9 @@
 //      point; the later of its two children's earliest points first shares
 //      a prefix of the node's length with an earlier point, which gives
 //      every L_v;
-//   4. the draws, one thread per generator in point order (the only serial
-//      step: numpy's SFC64 stream and its bounded-integer rule);
+//   4. the draws: how many outputs each takes from the generator (prefix
+//      counts), the streams (the only serial step: numpy's SFC64), and the
+//      draws' bits from them, by numpy's bounded-integer rule;
 //   5. each node's part of the scramble (its earliest point's draw over the
 //      depths the node spans) and each leaf's OR over its ancestors;
 //   6. xrb = (xb << (tmax_new - tmax)) ^ scramble, transposed back.
@@ -72,141 +73,222 @@ __global__ void nus_keys_kernel(NusDims m, const u64 *__restrict__ xb, const u64
 
 // ---- 2-3. the radix sort and the bottom-up tree pass: nus_dev.cuh -------------------
 
-// ---- 4. the draws, one thread per generator --------------------------------------
-// One thread per generator, 32 generators (rows of the draw array) per warp.  L_v
-// comes in 16 at a time (one 16-byte load per group, rows start 16-byte aligned),
-// three groups ahead of the draws.  A group whose 16 draws are all 64-bit draws
-// (33..63 bits) or all 32-bit draws (1..32 bits), the usual case, runs unrolled
-// without a branch per draw, its draws kept in registers; the warp then writes
-// every such row's 128 bytes through shared memory, each 16-byte store
-// instruction covering four rows' whole lines (a thread storing its own row would
-// touch 32 lines per instruction).  Any other group (the first and last, repeated
-// keys, mixed widths) takes the general path and stores its draws one by one.
+// ---- 4. the draws ------------------------------------------------------------------
+// Point v's draw of nb = T - 1 - L_v bits (the phantom's of T, first of all) is, by numpy's rules, the
+// top nb bits of one 64-bit output (nb > 32), or of a 32-bit half (0 < nb <= 32): the high half kept
+// from the last output that a half draw took, else the low half of a new output, whose high half is
+// then kept.  So half draws alternate between a new output and the kept half, and the outputs taken
+// before a draw are the full draws before it plus every other half draw: prefix counts.  The counts
+// come first (one warp per 256 points, then a scan per generator); the stream itself, the only
+// serial part, then runs without looking at the draws; and the draws take their bits from it, a
+// thread per point.  With the draws formatted and stored inside the serial loop, a step took
+// 68 cycles; the bare chain of 64-bit integer operations takes about 30 on one warp (32
+// generators).  r=4, d=8, n=200000: 7.15 ms for the draws before, 2.99 now (stream 2.93, 28 cycles a step).
 
-// the top nb bits (33 <= nb <= 63) of a 64-bit output: a right shift by 64 - nb < 32
-__device__ __forceinline__ u64 top_bits64(u64 x, u32 nb)
+constexpr u32 DT = 256;  // points per warp of the counting and formatting passes: all loads in flight at once
+
+// A tile's draws of more than 32 bits and of 1 to 32, with the full draws before its last two half
+// draws; after the scan the prefix counts up to and including the tile, and in last1 the output
+// that the last half draw with a new one took (NONE: no such draw).
+struct DrawCount {
+    u32 full, half, last1, last2;
+};
+
+// a generator's stream: outputs to run, and numpy's kept half at the start
+struct DrawInfo {
+    u32 outputs, has, half, pad;
+};
+
+__device__ __forceinline__ u32 tiles_of_draws(u32 N) { return (N + DT - 1) / DT; }
+
+// bits that point v draws
+__device__ __forceinline__ u32 draw_bits(const NusDims &m, u32 v, u32 L)
 {
-    const u32 sh = 64u - nb, lo = (u32)x, hi = (u32)(x >> 32);
-    return ((u64)(hi >> sh) << 32) | __funnelshift_r(lo, hi, sh);
+    if (v < m.H0) return m.fresh ? m.T : 0u;
+    return L + 1 >= m.T ? 0u : m.T - 1 - L;
 }
 
-__device__ __forceinline__ u32 byte_of(const u32 (&w)[4], int e) { return (w[e >> 2] >> (8 * (e & 3))) & 255u; }
-
-__device__ __forceinline__ u32 max_byte(const uint4 &c)
+// the same for a lane's points v0, v0 + 32, .. of a tile; 0 past the end
+__device__ __forceinline__ void tile_bits(const NusDims &m, const unsigned char *__restrict__ L, u32 v0,
+                                          u32 (&nb)[DT / 32])
 {
-    const u32 m4 = __vmaxu4(__vmaxu4(c.x, c.y), __vmaxu4(c.z, c.w));
-    return max(max(m4 & 255u, (m4 >> 8) & 255u), max((m4 >> 16) & 255u, m4 >> 24));
+#pragma unroll
+    for (u32 i = 0; i < DT / 32; i++) nb[i] = v0 + 32 * i < m.N && v0 + 32 * i >= m.H0 ? L[v0 + 32 * i] : 0;
+#pragma unroll
+    for (u32 i = 0; i < DT / 32; i++) nb[i] = v0 + 32 * i < m.N ? draw_bits(m, v0 + 32 * i, nb[i]) : 0;
 }
 
-__device__ __forceinline__ u32 min_byte(const uint4 &c)
-{
-    const u32 m4 = __vminu4(__vminu4(c.x, c.y), __vminu4(c.z, c.w));
-    return min(min(m4 & 255u, (m4 >> 8) & 255u), min((m4 >> 16) & 255u, m4 >> 24));
-}
+// outputs that the first h half draws take, `has`: a half was kept at the start
+__device__ __forceinline__ u32 half_outputs(u32 h, u32 has) { return (h + 1 - has) >> 1; }
 
-constexpr int DRAW_AHEAD = 4;
-
-__global__ void __launch_bounds__(32) nus_draw_kernel(NusDims m, u64 *__restrict__ states,
-                                                      const unsigned char *__restrict__ Lv, u64 *__restrict__ draw)
+__global__ void __launch_bounds__(256) nus_draw_count_kernel(NusDims m, const unsigned char *__restrict__ Lv,
+                                                             DrawCount *__restrict__ counts)
 {
-    // a warp's 32 rows of one group, 128 bytes each plus 16 of padding (the rows' 16-byte
-    // chunks then fall in different banks)
-    __shared__ uint4 stage[32][9];
-    const u32 lane = threadIdx.x, g0 = blockIdx.x * 32, g = g0 + lane;
-    const bool active = g < m.S;  // lanes past the last generator stay for the warp's stores
-    u64 *st = states + (u64)(active ? m.s0 + g : 0) * 6;
-    Sfc64 r{0, 0, 0, 0, 0, 0};
-    if (active) r = Sfc64{st[0], st[1], st[2], st[3], st[5], (u32)(st[4] != 0)};
-    const u64 off = (u64)(active ? g : 0) * m.NP;
-    const int T = (int)m.T;
-    u64 *D = draw + off;
-    if (active && m.fresh) D[0] = r.bits((u32)T);
-    const uint4 *L4 = reinterpret_cast<const uint4 *>(Lv + off);
-    const u32 gend = (m.N + 15) >> 4;  // groups covering [0, N); NP keeps the last one in the row
-    u32 gq = m.H0 >> 4;
-    uint4 ring[DRAW_AHEAD];
+    const u32 lane = threadIdx.x & 31, tile = blockIdx.x * 8 + (threadIdx.x >> 5), g = blockIdx.y;
+    const u32 tiles = tiles_of_draws(m.N);
+    if (tile >= tiles) return;
+    u32 nb[DT / 32];
+    tile_bits(m, Lv + (u64)g * m.NP, tile * DT + lane, nb);
+    DrawCount c{0, 0, 0, 0};
 #pragma unroll
-    for (int k = 0; k < DRAW_AHEAD; k++)
-        ring[k] = (active && gq + k < gend) ? L4[gq + k] : make_uint4(0, 0, 0, 0);
-    for (; gq < gend; gq++) {  // the same groups in every lane
-        const uint4 cur = ring[0];
-#pragma unroll
-        for (int k = 0; k < DRAW_AHEAD - 1; k++) ring[k] = ring[k + 1];
-        ring[DRAW_AHEAD - 1] = (active && gq + DRAW_AHEAD < gend) ? L4[gq + DRAW_AHEAD] : make_uint4(0, 0, 0, 0);
-        const u32 w[4] = {cur.x, cur.y, cur.z, cur.w};
-        const u32 v0 = gq << 4;
-        const bool inside = active && v0 >= m.H0 && v0 + 16 <= m.N;
-        const int lmax = (int)max_byte(cur), lmin = (int)min_byte(cur);
-        u64 y[16];
-        bool staged = false;
-        if (inside && lmax <= T - 34) {  // 16 draws of T-1-L in [33, 63] bits
-#pragma unroll
-            for (int e = 0; e < 16; e++) y[e] = top_bits64(r.next64(), (u32)(T - 1) - byte_of(w, e));
-            staged = true;
-        } else if (inside && lmin >= T - 33 && lmax <= T - 2) {  // 16 draws of 1..32 bits
-            // a draw of nb bits is the top nb bits of a 32-bit half: numpy's buffered half first,
-            // then both halves of each output, low first; the last output's high half is kept
-#define NUS_SH(e) (32u - ((u32)(T - 1) - byte_of(w, (e))))
-            if (r.has) {
-                y[0] = (u32)r.half >> NUS_SH(0);
-#pragma unroll
-                for (int e = 1; e < 15; e += 2) {
-                    const u64 x = r.next64();
-                    y[e] = (u32)x >> NUS_SH(e);
-                    y[e + 1] = (u32)(x >> 32) >> NUS_SH(e + 1);
-                }
-                const u64 x = r.next64();
-                y[15] = (u32)x >> NUS_SH(15);
-                r.half = x >> 32;
-                r.has = 1;
-            } else {
-#pragma unroll
-                for (int e = 0; e < 16; e += 2) {
-                    const u64 x = r.next64();
-                    y[e] = (u32)x >> NUS_SH(e);
-                    y[e + 1] = (u32)(x >> 32) >> NUS_SH(e + 1);
-                    r.half = x >> 32;
-                }
-            }
-#undef NUS_SH
-            staged = true;
-        } else if (active) {
-#pragma unroll 1
-            for (int e = 0; e < 16; e++) {
-                const u32 v = v0 + e;
-                if (v >= m.H0 && v < m.N) {
-                    const int L = (int)byte_of(w, e);
-                    D[v] = r.bits(L >= T - 1 ? 0u : (u32)(T - 1 - L));
-                }
-            }
+    for (u32 i = 0; i < DT / 32; i++) {
+        const u32 full = __ballot_sync(0xFFFFFFFFu, nb[i] > 32);
+        const u32 half = __ballot_sync(0xFFFFFFFFu, nb[i] && nb[i] <= 32);
+        if (half) {
+            const u32 top = 1u << (31 - __clz(half)), rest = half ^ top;
+            c.last2 = rest ? c.full + __popc(full & ((1u << (31 - __clz(rest))) - 1)) : c.last1;
+            c.last1 = c.full + __popc(full & (top - 1));
         }
-        if (staged) {
-#pragma unroll
-            for (int c = 0; c < 8; c++)
-                stage[lane][c] = make_uint4((u32)y[2 * c], (u32)(y[2 * c] >> 32), (u32)y[2 * c + 1],
-                                            (u32)(y[2 * c + 1] >> 32));
-        }
-        const u32 rows = __ballot_sync(0xFFFFFFFFu, staged);
-        __syncwarp();
-        if (rows) {
-            // store i: rows 4i .. 4i+3, eight lanes (16 bytes each) per row
-            const u32 c = lane & 7;
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                const u32 R = 4 * i + (lane >> 3);
-                if ((rows >> R) & 1u)
-                    *reinterpret_cast<uint4 *>(draw + (u64)(g0 + R) * m.NP + v0 + 2 * c) = stage[R][c];
-            }
-        }
-        __syncwarp();
+        c.full += __popc(full);
+        c.half += __popc(half);
     }
-    if (!active) return;
-    st[0] = r.a;
-    st[1] = r.b;
-    st[2] = r.c;
-    st[3] = r.w;
-    st[4] = r.has;
-    st[5] = r.half;  // numpy keeps the last buffered half here, used or not
+    if (lane == 0) counts[(u64)g * tiles + tile] = c;
+}
+
+// one warp per generator: the scan over its tiles, the stream's length
+__global__ void __launch_bounds__(32) nus_draw_scan_kernel(NusDims m, const u64 *__restrict__ states,
+                                                           DrawCount *__restrict__ counts, DrawInfo *__restrict__ info)
+{
+    const u32 lane = threadIdx.x, g = blockIdx.x, tiles = tiles_of_draws(m.N);
+    const u64 *st = states + (m.s0 + g) * 6;
+    const u32 has = st[4] != 0;
+    DrawCount *C = counts + (u64)g * tiles;
+    u32 full = 0, half = 0, kept = NONE;
+    for (u32 t0 = 0; t0 < tiles; t0 += 32) {
+        const u32 t = t0 + lane;
+        const DrawCount c = t < tiles ? C[t] : DrawCount{0, 0, 0, 0};
+        u32 f = c.full, h = c.half;
+#pragma unroll
+        for (u32 o = 1; o < 32; o *= 2) {
+            const u32 a = __shfl_up_sync(0xFFFFFFFFu, f, o), b = __shfl_up_sync(0xFFFFFFFFu, h, o);
+            if (lane >= o) {
+                f += a;
+                h += b;
+            }
+        }
+        // this tile's last half draw with a new output: its last one or the one before, by parity
+        const u32 before = full + f - c.full, end = half + h;  // end: half draws up to and including the tile
+        const u32 odd = (end - 1 + has) & 1u;                  // the last one took the kept half
+        const bool any = c.half > odd;
+        const u32 mine = before + (odd ? c.last2 : c.last1) + half_outputs(end - 1 - odd, has);
+        const u32 with = __ballot_sync(0xFFFFFFFFu, any) & (0xFFFFFFFFu >> (31 - lane));
+        const u32 from = __shfl_sync(0xFFFFFFFFu, mine, with ? 31 - __clz(with) : 0);
+        const u32 k = with ? from : kept;
+        if (t < tiles) C[t] = DrawCount{full + f, end, k, 0};
+        full += __shfl_sync(0xFFFFFFFFu, f, 31);
+        half += __shfl_sync(0xFFFFFFFFu, h, 31);
+        kept = __shfl_sync(0xFFFFFFFFu, k, 31);
+    }
+    if (lane == 0) info[g] = DrawInfo{full + half_outputs(half, has), has, (u32)st[5], 0};
+}
+
+constexpr u32 STREAM_STEPS = 32;  // outputs per generator between two barriers
+
+// The streams of 32 generators: warp 0, alone on its quarter of the SM, steps them (a lane each) into
+// shared memory, the other three warps write whole 256-byte row segments behind it.
+__global__ void __launch_bounds__(128) nus_stream_kernel(NusDims m, u64 *__restrict__ states,
+                                                         const DrawInfo *__restrict__ info, u64 *__restrict__ raw)
+{
+    __shared__ u64 buf[2][STREAM_STEPS][33];
+    const u32 warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g0 = blockIdx.x * 32, g = g0 + lane;
+    const u32 need = g < m.S ? info[g].outputs : 0;
+    const u32 most = __reduce_max_sync(0xFFFFFFFFu, need), least = __reduce_min_sync(0xFFFFFFFFu, need);
+    u64 *st = states + (g < m.S ? m.s0 + g : 0) * 6;
+    Sfc64 r{0, 0, 0, 0, 0, 0};
+    if (warp == 0 && g < m.S) r = Sfc64{st[0], st[1], st[2], st[3], 0, 0};
+    for (u32 i0 = 0, k = 0; i0 < most; i0 += STREAM_STEPS, k ^= 1) {
+        if (warp == 0) {
+            if (i0 + STREAM_STEPS <= least) {
+#pragma unroll
+                for (u32 s = 0; s < STREAM_STEPS; s++) buf[k][s][lane] = r.next64();
+            } else {
+                for (u32 s = 0; s < STREAM_STEPS && i0 + s < need; s++) buf[k][s][lane] = r.next64();
+            }
+        }
+        __syncthreads();  // also: the other warps are done with the other buffer
+        if (warp != 0) {
+            // all reads ahead of all stores: row by row, three warps took longer than the 32 steps
+            u64 x[11];
+#pragma unroll
+            for (u32 e = 0; e < 11; e++) x[e] = buf[k][lane][min(warp - 1 + 3 * e, 31u)];
+            u64 *row = raw + (u64)(g0 + warp - 1) * m.NP + i0 + lane;
+#pragma unroll
+            for (u32 e = 0; e < 11; e++) {
+                const u32 q = warp - 1 + 3 * e, end = __shfl_sync(0xFFFFFFFFu, need, q & 31u);
+                if (q < 32 && i0 + lane < end) row[(u64)(3 * e) * m.NP] = x[e];
+            }
+        }
+    }
+    if (warp == 0 && g < m.S) {
+        st[0] = r.a;
+        st[1] = r.b;
+        st[2] = r.c;
+        st[3] = r.w;
+    }
+}
+
+// the draws of a tile from the stream; the last tile leaves numpy's kept half in the state
+__global__ void __launch_bounds__(256) nus_draw_kernel(NusDims m, const unsigned char *__restrict__ Lv,
+                                                       const DrawCount *__restrict__ counts,
+                                                       const DrawInfo *__restrict__ info, const u64 *__restrict__ raw,
+                                                       u64 *__restrict__ states, u64 *__restrict__ draw)
+{
+    const u32 lane = threadIdx.x & 31, tile = blockIdx.x * 8 + (threadIdx.x >> 5), g = blockIdx.y;
+    const u32 tiles = tiles_of_draws(m.N);
+    if (tile >= tiles) return;
+    const u64 *R = raw + (u64)g * m.NP;
+    u64 *D = draw + (u64)g * m.NP;
+    const DrawInfo in = info[g];
+    const u32 v0 = tile * DT + lane;
+    u32 nb[DT / 32], at[DT / 32];  // at: the output, NONE for the state's half
+    u32 high = 0;                  // bit i: draw i takes a kept half
+    tile_bits(m, Lv + (u64)g * m.NP, v0, nb);
+    DrawCount c{0, 0, NONE, 0};
+    if (tile) c = counts[(u64)g * tiles + tile - 1];
+    u32 kept = c.last1;  // the output whose high half is or was kept last (NONE: the state's own half)
+    const u32 lt = (1u << lane) - 1;
+#pragma unroll
+    for (u32 i = 0; i < DT / 32; i++) {
+        const bool is_half = nb[i] && nb[i] <= 32;
+        const u32 full = __ballot_sync(0xFFFFFFFFu, nb[i] > 32), half = __ballot_sync(0xFFFFFFFFu, is_half);
+        at[i] = c.full + __popc(full & lt);
+        if (half) {  // the same for the warp
+            const u32 h = c.half + __popc(half & lt);  // half draws before this point
+            at[i] += half_outputs(h, in.has);
+            const bool fresh = ((h + in.has) & 1u) == 0;
+            const u32 news = __ballot_sync(0xFFFFFFFFu, is_half && fresh), before = news & lt;
+            // the last new output of a half draw before each lane
+            const u32 from = __shfl_sync(0xFFFFFFFFu, at[i], before ? 31 - __clz(before) : 0);
+            const u32 last = __shfl_sync(0xFFFFFFFFu, at[i], news ? 31 - __clz(news) : 0);
+            if (is_half && !fresh) {
+                at[i] = before ? from : kept;
+                high |= 1u << i;
+            }
+            if (news) kept = last;
+        } else {
+            at[i] += half_outputs(c.half, in.has);
+        }
+        c.full += __popc(full);
+        c.half += __popc(half);
+    }
+    u64 x[DT / 32];
+#pragma unroll
+    for (u32 i = 0; i < DT / 32; i++) x[i] = nb[i] && at[i] != NONE ? R[at[i]] : (u64)in.half << 32;
+#pragma unroll
+    for (u32 i = 0; i < DT / 32; i++) {
+        const u32 v = v0 + 32 * i;
+        u64 y = 0;
+        if (nb[i] > 32)
+            y = nb[i] == 64 ? x[i] : x[i] >> (64 - nb[i]);
+        else if (nb[i])
+            y = ((high >> i) & 1u ? (u32)(x[i] >> 32) : (u32)x[i]) >> (32 - nb[i]);
+        if (v < m.N && (v >= m.H0 || m.fresh)) D[v] = y;
+    }
+    if (tile == tiles - 1 && lane == 0) {
+        u64 *st = states + (m.s0 + g) * 6;
+        st[4] = (in.has + c.half) & 1u;
+        st[5] = kept == NONE ? in.half : R[kept] >> 32;  // numpy keeps the last kept half here, used or not
+    }
 }
 
 // ---- 5. scramble bits: each node's band, each leaf's ancestors -----------------
@@ -468,7 +550,16 @@ int qmc_dnb2_nested_uniform_scramble(uint64_t r, uint64_t n, uint64_t d, uint64_
             rc = qmcgb::launch_status("dnb2_nus tree");
             if (rc) return rc;
         }
-        nus_draw_kernel<<<(m.S + 31) / 32, 32, 0, st>>>(m, st_, w.Lv, w.draw);
+        // the counts and stream lengths in the sort's count array, the outputs in the array that the
+        // scrambles take later
+        const u32 dt = (m.N + DT - 1) / DT;
+        DrawInfo *info = (DrawInfo *)w.cnt;
+        DrawCount *counts = (DrawCount *)w.cnt + m.S;
+        const dim3 dg((dt + 7) / 8, m.S);
+        nus_draw_count_kernel<<<dg, 256, 0, st>>>(m, w.Lv, counts);
+        nus_draw_scan_kernel<<<m.S, 32, 0, st>>>(m, st_, counts, info);
+        nus_stream_kernel<<<(m.S + 31) / 32, 128, 0, st>>>(m, st_, info, w.shv);
+        nus_draw_kernel<<<dg, 256, 0, st>>>(m, w.Lv, counts, info, w.shv, st_, w.draw);
         rc = qmcgb::launch_status("dnb2_nus draws");
         if (rc) return rc;
         if (draws_out) {
