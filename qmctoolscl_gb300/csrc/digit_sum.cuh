@@ -90,4 +90,58 @@ DS_HD u64 mul_small(u64 r, u32 m)
     return ((r >> 52) + 10u - lz) * HIDDEN + mant + up;
 }
 
+// Sums in integers.  While a sum v stays in its binade (last place 2^(E - 1075)), RN(v + y) adds y
+// rounded to that place, whatever v is, but for ties.  With y as F = floor(y * 2^unit) and
+// s = unit - 53 - tiny, tiny = 1022 - E (v in [2^-(tiny+1), 2^-tiny)), the rounded terms add up in
+//     acc = (acc + F + half) & ~(2^s - 1),  half = 2^(s-1),
+// and r = acc >> s is added to v's bits at last: a carry into the exponent shows that v left its
+// binade.  Terms that can tie take the even place: v's last bit in acc, a sticky bit in F.
+
+// floor(y * 2^unit) for the bits y of a non-negative double below 2^(63 - unit) (so that a sum of such
+// terms, at most that bound in all, has room to round up); *exact: nothing cut off
+DS_HD u64 fixed_term(u64 y, int unit, bool *exact)
+{
+    const u32 e = (u32)(y >> 52);
+    *exact = true;
+    if (!e) {
+        *exact = y == 0;
+        return 0;
+    }
+    const u64 m = (y & FRAC) | HIDDEN;
+    const int sh = (int)e - (1075 - unit);
+    if (sh >= 0) return m << sh;
+    if (sh <= -53) {
+        *exact = false;
+        return 0;
+    }
+    const u64 F = m >> -sh;
+    *exact = F << -sh == m;
+    return F;
+}
+
+// whether F (exact) ties for some v with tiny <= most
+DS_HD bool can_tie(u64 F, bool exact, int unit, int most)
+{
+    if (!exact || !F) return false;
+#ifdef __CUDA_ARCH__
+    const int z = __ffsll((long long)F) - 1;
+#else
+    const int z = __builtin_ctzll(F);
+#endif
+    return z < unit - 53 && z >= unit - 54 - most;  // the lowest bit is half a last place for s = z + 1
+}
+
+DS_HD u64 add_plain(u64 acc, u64 F, u32 half)
+{
+    const u64 a = acc + F + half;
+    return (a & 0xFFFFFFFF00000000ull) | ((u32)a & (0u - 2 * half));
+}
+
+DS_HD u64 add_even(u64 acc, u64 F, u32 half)
+{
+    u64 a = acc + F;
+    a += half - 1 + (((u32)a & (2 * half)) ? 1u : 0u);
+    return (a & 0xFFFFFFFF00000000ull) | ((u32)a & (0u - 2 * half));
+}
+
 }  // namespace dsum

@@ -754,13 +754,232 @@ constexpr u32 I2F_TMAX = 64;            // recip table depth held in shared memo
 constexpr u32 I2F_SMEM_WORDS = 2048;    // dynamic shared memory (16 KB, 8 CTAs per SM): term or recip table
 enum I2fMode { I2F_LOOP = 0, I2F_RECIP = 1, I2F_TERMS = 2 };
 
+// ---- 16 digits and more: staged digits, the sum mostly in integers (digit_sum.cuh)
+
+constexpr u32 I2F_STAGED = 16;
+
+constexpr int I2F_HEAD_BITS = 13;           // rows before b^t1 >= 2^13 add on the FP64 unit
+constexpr int I2F_UNIT = 63 + I2F_HEAD_BITS;  // the integer rows' terms sum to 2^63 at most
+constexpr int I2F_TINY = 9;                 // the integer rows need a sum of at least 2^-10
+
+// a dimension's table: rows t < t1 hold RN(recip_t * dg) as doubles, the others F; rows t1 .. tr-1
+// have terms that can tie
+struct I2fDim {
+    u32 b, t1, tr, off;
+};
+
+constexpr u32 I2F_CTAS = 2;               // per SM (3 with 8 digits at a time: 244 us for 229)
+constexpr u32 I2F_CHUNK = 16;             // digits of a point copied at a time: a line
+constexpr u32 I2F_ROW = I2F_CHUNK * 8 + 16;  // and its place in a warp's buffer (padded: no bank conflicts)
+constexpr u32 I2F_BUF = 32 * I2F_ROW;
+
+// Digits t0 .. t0+15 (below tmax) of `points` points, `row` words apart, into the warp's buffer, whole
+// lines by consecutive lanes (a lane reading its own point's digits touches 32 lines per load).
+__device__ __forceinline__ void copy_digits(const u64 *dig, u64 row, u32 points, u32 t0, u32 tmax, u32 buf)
+{
+    const u32 lane = threadIdx.x % 32, cnt = min(I2F_CHUNK, tmax - t0);
+    if ((tmax & 1) == 0 && ((uintptr_t)dig & 15) == 0) {  // then every pair of digits is 16-byte aligned
+        const u32 k = lane % (I2F_CHUNK / 2);
+#pragma unroll
+        for (u32 u = 0; u < I2F_CHUNK / 2; u++) {
+            const u32 p = (64 / I2F_CHUNK) * u + lane / (I2F_CHUNK / 2);
+            if (p < points && 2 * k < cnt)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(buf + p * I2F_ROW + 16 * k),
+                             "l"(dig + p * row + t0 + 2 * k));
+        }
+    } else {
+        const u32 k = lane % I2F_CHUNK;
+#pragma unroll
+        for (u32 u = 0; u < I2F_CHUNK; u++) {
+            const u32 p = (32 / I2F_CHUNK) * u + lane / I2F_CHUNK;
+            if (p < points && k < cnt)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(buf + p * I2F_ROW + 8 * k),
+                             "l"(dig + p * row + t0 + k));
+        }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// The running sum of one point.
+struct I2fSum {
+    double v;
+    u64 acc;
+    u32 half, beyond, tiny;
+};
+
+// digits t0 .. t0+15 of the lane's point
+__device__ __forceinline__ void add_digits(I2fSum &S, const u64 *T, const I2fDim &D, const unsigned char *dig, u32 t0,
+                                           u32 tmax)
+{
+#pragma unroll 1
+    for (u32 h = 0; h < I2F_CHUNK && t0 + h < tmax; h += 8) {
+        u64 y[8];
+#pragma unroll
+        for (u32 u = 0; u < 8; u += 2) {
+            const uint4 q = *(const uint4 *)(dig + 8 * (h + u));
+            const u32 lo[2] = {q.x, q.z}, hi[2] = {q.y, q.w};
+#pragma unroll
+            for (u32 e = 0; e < 2; e++) {
+                if (t0 + h + u + e >= tmax) continue;  // the same for the warp
+                const u32 idx = min(lo[e], D.b - 1);
+                S.beyond |= hi[e] | (lo[e] ^ idx);
+                y[u + e] = T[(t0 + h + u + e) * D.b + idx];
+            }
+        }
+        // the sections too are the same for the whole warp: it owns a dimension
+        if (t0 + h >= D.tr && t0 + h + 8 <= tmax) {
+#pragma unroll
+            for (u32 u = 0; u < 8; u++) S.acc = dsum::add_plain(S.acc, y[u], S.half);
+            continue;
+        }
+#pragma unroll
+        for (u32 u = 0; u < 8; u++) {
+            const u32 t = t0 + h + u;
+            if (t >= tmax) break;
+            if (t < D.t1) {
+                S.v = __dadd_rn(S.v, as_double(y[u]));  // gdn_integer_to_float.c:37
+                if (t + 1 == D.t1) {
+                    S.tiny = 1022u - (u32)(as_bits(S.v) >> 52);
+                    const u32 s = (u32)(I2F_UNIT - 53) - (S.tiny <= (u32)I2F_TINY ? S.tiny : 0u);
+                    S.half = 1u << (s - 1);
+                    S.acc = (as_bits(S.v) & 1) << s;
+                }
+            } else if (t < D.tr) {
+                S.acc = dsum::add_even(S.acc, y[u], S.half);
+            } else {
+                S.acc = dsum::add_plain(S.acc, y[u], S.half);
+            }
+        }
+    }
+}
+
+// The point's value; false where it is to be redone: a digit at or above the base, a sum below 2^-10
+// after t1 rows, or one that left its binade.
+__device__ __forceinline__ bool end_digits(const I2fSum &S, const I2fDim &D, u32 tmax, double *out)
+{
+    *out = S.v;
+    if (D.t1 >= tmax) return !S.beyond;
+    const u64 vb = as_bits(S.v), r = (vb & ~1ull) + (S.acc >> (32 - __clz((int)S.half)));
+    *out = as_double(r);
+    return !S.beyond && S.tiny <= (u32)I2F_TINY && (r >> 52) == (vb >> 52);
+}
+
+// words of a CTA's recip table, whole 16-byte units
+__host__ __device__ __forceinline__ u32 i2f_recip_words(u64 d, u64 tmax)
+{
+    return ((u32)((d < I2F_DIMS ? d : I2F_DIMS) * (tmax < I2F_TMAX ? tmax : I2F_TMAX)) + 1) & ~1u;
+}
+
+// Offsets of the term tables -- RN(recip_t * dg) for t < tmax, dg < b -- of a CTA's dimensions, by one
+// thread; false when they do not fit I2F_SMEM_WORDS together.
+__device__ bool i2f_tables(const u64 *bl, u32 nd, u64 tmax, I2fDim *dims)
+{
+    u64 acc = 0;
+    bool fits = tmax <= I2F_TMAX;
+    for (u32 c = 0; c < nd && fits; c++) {
+        const u64 b = bl[c];
+        fits = b >= 2 && b <= I2F_SMEM_WORDS;
+        u32 t1 = 1;
+        for (u64 v = b; fits && v < (1ull << I2F_HEAD_BITS) && t1 < tmax; v *= b) t1++;
+        if (dims) dims[c] = I2fDim{(u32)b, t1, t1, (u32)acc};
+        acc += tmax * b;
+        fits = fits && acc <= I2F_SMEM_WORDS;
+    }
+    return fits;
+}
+
+// 16 to 64 digits, term tables that fit I2F_SMEM_WORDS (the others are left to gdn_to_float_kernel).  Each CTA
+// converts a run of points for up to 32 dimensions: a warp takes 32 points of one dimension after
+// another, 16 digits at a time, the next 16 on their way to shared memory; the products come from the
+// tables and the sum from integers after the first rows.  d=4, bases 2, 3, 5, 7, tmax=32, 2^20 points:
+// 358 us with an FP64 add per digit (the unit 83 % busy) and each lane reading its own point, 229
+// now (ALU 35 %, FP64 31 %: 16 warps per SM wait for one another's phases).  One wave of CTAs: the tables (a serial
+// chain of divides) cost as much as 500 points.  Below 16 digits a unit is too short to hide its
+// copies (base 541, 8 digits: 163 us without, 202 with).
+__global__ void __launch_bounds__(THREADS, I2F_CTAS)
+    gdn_terms_float_kernel(u64 r, u64 n, u64 d, u64 r_b, u64 tmax, const u64 *bases, const u64 *xdig, double *x,
+                           u64 rows_per_cta, u32 dim_tiles, u64 l_off)
+{
+    extern __shared__ __align__(16) double i2f_sm[];
+    __shared__ I2fDim dims[I2F_DIMS];
+    __shared__ u32 fits;
+    const u64 l = l_off + (u64)blockIdx.y / dim_tiles;
+    if (l >= r) return;
+    const u64 j0 = (u64)(blockIdx.y % dim_tiles) * I2F_DIMS;
+    const u32 nd = (u32)min((u64)I2F_DIMS, d - j0);
+    const u64 *bl = bases + (l % r_b) * d + j0;
+    double *recips = i2f_sm + I2F_SMEM_WORDS;
+    if (threadIdx.x == 0) fits = i2f_tables(bl, nd, tmax, dims);
+    __syncthreads();
+    if (!fits) return;
+    for (u32 c = threadIdx.x; c < nd; c += blockDim.x) fill_recips(recips + c * tmax, bl[c], tmax);
+    __syncthreads();
+    for (u32 c = 0; c < nd; c++) {
+        const u32 b = dims[c].b, t1 = dims[c].t1, cnt = (u32)tmax * b;
+        u64 *T = (u64 *)i2f_sm + dims[c].off;
+        for (u32 k = threadIdx.x; k < cnt; k += blockDim.x) {
+            const u32 t = k / b, dg = k - t * b;
+            const u64 y = as_bits(__dmul_rn(recips[c * tmax + t], (double)dg));
+            T[k] = y;
+            if (t < t1) continue;
+            bool exact;
+            const u64 F = dsum::fixed_term(y, I2F_UNIT, &exact);
+            T[k] = F | (exact ? 0u : 1u);
+            if (dsum::can_tie(F, exact, I2F_UNIT, I2F_TINY)) atomicMax(&dims[c].tr, t + 1);
+        }
+    }
+    __syncthreads();
+    const u64 row0 = (u64)blockIdx.x * rows_per_cta;
+    if (row0 >= n) return;
+    const u64 rows = min(rows_per_cta, n - row0);
+    const u64 *xl = xdig + l * n * d * tmax;
+    const u32 lane = threadIdx.x % 32, warp = threadIdx.x / 32, units = (u32)((rows + 31) / 32) * nd;
+    const Div32 dv_nd = div32_dev(nd);
+    unsigned char *buf = (unsigned char *)(recips + i2f_recip_words(d, tmax)) + warp * (2 * I2F_BUF);
+    const u32 buf_a = (u32)__cvta_generic_to_shared(buf);
+    auto start = [&](u32 u, u32 t0, u32 k) {
+        if (u >= units) {
+            asm volatile("cp.async.commit_group;" ::: "memory");  // empty: the count of groups stays right
+            return;
+        }
+        const u32 rb = div32(dv_nd, u), c = u - rb * nd;
+        copy_digits(xl + ((row0 + rb * 32) * d + j0 + c) * tmax, d * tmax, (u32)min((u64)32, rows - rb * 32), t0,
+                    (u32)tmax, buf_a + k * I2F_BUF);
+    };
+    u32 k = 0;
+    if (tmax) start(warp, 0, 0);
+    for (u32 u = warp; u < units; u += THREADS / 32) {
+        const u32 rb = div32(dv_nd, u), c = u - rb * nd;
+        const I2fDim D = dims[c];
+        const u64 *T = (const u64 *)i2f_sm + D.off;
+        I2fSum S{0.0, 0, 1, 0, 0};
+        for (u32 t0 = 0; t0 < (u32)tmax; t0 += I2F_CHUNK) {
+            const bool last = t0 + I2F_CHUNK >= (u32)tmax;
+            start(last ? u + THREADS / 32 : u, last ? 0 : t0 + I2F_CHUNK, k ^ 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncwarp();
+            add_digits(S, T, D, buf + k * I2F_BUF + lane * I2F_ROW, t0, (u32)tmax);
+            __syncwarp();  // all have read before the buffer is filled again
+            k ^= 1;
+        }
+        const u64 i = row0 + rb * 32 + lane, j = j0 + c;
+        if (i >= row0 + rows) continue;
+        double v;
+        if (!end_digits(S, D, (u32)tmax, &v)) v = digits_to_double(recips + c * tmax, xl + (i * d + j) * tmax, tmax);
+        x[l * n * d + i * d + j] = v;
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
 // Each CTA converts a run of points for up to 32 dimensions.  When the CTA's
 // term tables -- RN(recip_t * dg) for t < tmax, dg < b, per dimension -- fit
 // in 16 KB, the products come from shared memory and only the adds run on the
-// FP64 unit; else a table of recip_t (tmax <= 64), else the reference's loop.
+// FP64 unit (tmax below 16; from there on gdn_terms_float_kernel has done them:
+// staged); else a table of recip_t (tmax <= 64), else the reference's loop.
 __global__ void __launch_bounds__(THREADS) gdn_to_float_kernel(u64 r, u64 n, u64 d, u64 r_b, u64 tmax,
                                                                const u64 *bases, const u64 *xdig, double *x,
-                                                               u64 rows_per_cta, u32 dim_tiles, u64 l_off)
+                                                               u64 rows_per_cta, u32 dim_tiles, u64 l_off,
+                                                               u32 staged)
 {
     extern __shared__ __align__(16) double i2f_sm[];
     __shared__ u32 toff[I2F_DIMS + 1], tb[I2F_DIMS], mode;
@@ -784,6 +1003,7 @@ __global__ void __launch_bounds__(THREADS) gdn_to_float_kernel(u64 r, u64 n, u64
         mode = fits ? I2F_TERMS : tmax <= I2F_TMAX ? I2F_RECIP : I2F_LOOP;
     }
     __syncthreads();
+    if (staged && mode == I2F_TERMS) return;  // gdn_terms_float_kernel has done these dimensions
     if (mode == I2F_TERMS) {
         // recip_t into column 1 of each row, then every entry from its row's recip
         for (u32 c = threadIdx.x; c < nd; c += blockDim.x) {
@@ -1071,11 +1291,27 @@ int qmc_gdn_integer_to_float(uint64_t r, uint64_t n, uint64_t d, uint64_t r_b, u
     if (r == 0 || n == 0 || d == 0) return QMC_OK;
     QMC_REQUIRE(r_b > 0 && bases && x && (tmax == 0 || xdig), "bad r_b or null array pointer");
     u64 splits;
+    // the smallest tables: base 2 in every dimension
+    const bool staged = tmax >= I2F_STAGED && tmax <= I2F_TMAX && tmax * 2 * (d < I2F_DIMS ? d : I2F_DIMS) <= I2F_SMEM_WORDS;
+    if (staged) {
+        const size_t smem = (I2F_SMEM_WORDS + i2f_recip_words(d, tmax)) * sizeof(double) + THREADS / 32 * 2 * I2F_BUF;
+        if (int rc = qmcgb::raise_smem_limit((const void *)gdn_terms_float_kernel, smem, "gdn_integer_to_float")) return rc;
+        PointGrid pg = point_grid(r, n, d, 1, I2F_DIMS, &splits, I2F_CTAS);
+        // one wave: a split less where the rounding up made it more
+        if (splits > 1 && splits * r * pg.dim_tiles > (u64)qmcgb::sm_count() * I2F_CTAS) splits--;
+        pg.rows_per_cta = (n + splits - 1) / splits;
+        if (int rc = launch_points(r, pg.dim_tiles, [&](u64 l0, unsigned cnt) {
+                gdn_terms_float_kernel<<<dim3((unsigned)splits, cnt, 1), THREADS, smem, QMC_STREAM(s)>>>(
+                    r, n, d, r_b, tmax, (const u64 *)bases, (const u64 *)xdig, x, pg.rows_per_cta, pg.dim_tiles, l0);
+            }, "gdn_integer_to_float"))
+            return rc;
+    }
     const PointGrid pg = point_grid(r, n, d, 1, I2F_DIMS, &splits, 16);
     return launch_points(r, pg.dim_tiles, [&](u64 l0, unsigned cnt) {
         gdn_to_float_kernel<<<dim3((unsigned)splits, cnt, 1), THREADS, I2F_SMEM_WORDS * sizeof(double),
                               QMC_STREAM(s)>>>(
-            r, n, d, r_b, tmax, (const u64 *)bases, (const u64 *)xdig, x, pg.rows_per_cta, pg.dim_tiles, l0);
+            r, n, d, r_b, tmax, (const u64 *)bases, (const u64 *)xdig, x, pg.rows_per_cta, pg.dim_tiles, l0,
+            staged ? 1u : 0u);
     }, "gdn_integer_to_float");
 }
 

@@ -4,9 +4,9 @@
 // The sum of gdn_integer_to_float.c:33-39, v = RN(v + y_t), in three sections per (l, j):
 //  * rows [0, t1), b^t1 >= 2^16: FP64 adds (the first is a load);
 //  * the other rows: v's binade E is known now, and a term y becomes the integer
-//    F = floor(y * 2^80).  While v stays in its binade, RN(v + y) adds y rounded to v's last
+//    F = floor(y * 2^79).  While v stays in its binade, RN(v + y) adds y rounded to v's last
 //    place 2^(E - 1075), whatever v is (ties aside), so the rounded terms are summed on their
-//    own: acc = (acc + F + half) & ~(2^s - 1), s = 27 - (1022 - E): three integer
+//    own: acc = (acc + F + half) & ~(2^s - 1), s = 26 - (1022 - E): three integer
 //    instructions a row where the FP64 add holds its narrow pipe for half a clock per SM.
 //    The sum of the rounded terms is at last added to v's bits.  Rows [t1, tr), up to the last
 //    one with a term that ties for some v of at least 2^-10 (terms above about 2^-25; every row of
@@ -37,7 +37,7 @@ constexpr u32 HR_PTS = 2;          // points of a lane: 32 apart
 constexpr u32 HR_THREADS = 1024;   // 64 registers: 8.0 ms; 768 threads 8.8, 4 points on 640 threads 9.0 (first 100
                                    // primes, r=32, n=2^18; 4 dimensions unrolled 8.9: instruction cache)
 constexpr u32 HR_TINY = 9;         // integer rows need v >= 2^-(HR_TINY + 1)
-constexpr u32 HR_UNIT = 80;        // F counts 2^-80
+constexpr int HR_UNIT = 79;        // F counts 2^-79: the integer rows' terms sum to 2^63 at most
 constexpr u32 HR_HEAD_BITS = 16;   // b^t1 >= 2^16
 // Below these the warp kernel, which has no tables to set up, finishes sooner.  us, warp kernel / this
 // one, (r, n, d): (16, 8192, 100) 336 / 502, (32, 16384, 20) 487 / 744, (8, 65536, 37) 672 / 720,
@@ -61,37 +61,14 @@ __device__ __forceinline__ u32 hr_info(u32 t1, u32 tr, u32 rows, bool low_table)
     return t1 | tr << 10 | rows << 20 | (low_table ? 1u << 31 : 0u);
 }
 
-// F = floor(y * 2^80) for 0 <= y < 2^-16; *exact: nothing was cut off
-__device__ __forceinline__ u64 hr_fixed(u64 y, bool *exact)
-{
-    const u32 e = (u32)(y >> 52);
-    *exact = true;
-    if (!e) {
-        *exact = y == 0;
-        return 0;
-    }
-    const u64 m = (y & dsum::FRAC) | dsum::HIDDEN;
-    const int sh = (int)e - (1075 - (int)HR_UNIT);
-    if (sh >= 0) return m << sh;
-    if (sh <= -53) {
-        *exact = false;
-        return 0;
-    }
-    const u64 F = m >> -sh;
-    *exact = F << -sh == m;
-    return F;
-}
-
 // row flags: 1 a term that ties for some v in [2^-(HR_TINY+1), 1), 2 a digit at or above its base
 __device__ __forceinline__ u32 hr_term_flags(u64 y, u64 dig, u64 b)
 {
     u32 f = dig >= b ? 2u : 0u;
     if ((y >> 52) < 1023 - HR_HEAD_BITS) {
         bool exact;
-        const u64 F = hr_fixed(y, &exact);
-        const int z = F ? __ffsll((long long)F) - 1 : 64;  // the lowest bit is half a last place for s = z + 1
-        const int s = HR_UNIT - 53;
-        if (exact && z < s && z >= s - 1 - (int)HR_TINY) f |= 1u;
+        const u64 F = dsum::fixed_term(y, HR_UNIT, &exact);
+        if (dsum::can_tie(F, exact, HR_UNIT, HR_TINY)) f |= 1u;
     } else {
         f |= 1u;  // too large for the integer rows
     }
@@ -217,32 +194,24 @@ __device__ __forceinline__ void hr_values(const HDigits<LOW> (&W)[HR_PTS], u32 T
     }
     if (t1 == rows) return;
     u64 acc[HR_PTS];
-    u32 half[HR_PTS], keep[HR_PTS];
+    u32 half[HR_PTS];
 #pragma unroll
     for (u32 p = 0; p < HR_PTS; p++) {
         const u32 hi = (u32)__double2hiint(v[p]), tiny = 1022u - (hi >> 20);  // v < 1
         const u32 s = (HR_UNIT - 53) - (tiny <= HR_TINY ? tiny : 0u);
         half[p] = 1u << (s - 1);
-        keep[p] = 0u - (half[p] << 1);
         acc[p] = (u64)((u32)__double2loint(v[p]) & 1u) << s;
     }
     for (; t < tr; t++) {
         T += b8;
 #pragma unroll
-        for (u32 p = 0; p < HR_PTS; p++) {
-            u64 a = acc[p] + hr_ld64(T + W[p].at(t, b8));
-            a += half[p] - 1 + (((u32)a & (half[p] << 1)) ? 1u : 0u);
-            acc[p] = (a & 0xFFFFFFFF00000000ull) | ((u32)a & keep[p]);
-        }
+        for (u32 p = 0; p < HR_PTS; p++) acc[p] = dsum::add_even(acc[p], hr_ld64(T + W[p].at(t, b8)), half[p]);
     }
 #pragma unroll 1
     for (; t < rows; t++) {
         T += b8;
 #pragma unroll
-        for (u32 p = 0; p < HR_PTS; p++) {
-            const u64 a = acc[p] + hr_ld64(T + W[p].at(t, b8)) + half[p];
-            acc[p] = (a & 0xFFFFFFFF00000000ull) | ((u32)a & keep[p]);
-        }
+        for (u32 p = 0; p < HR_PTS; p++) acc[p] = dsum::add_plain(acc[p], hr_ld64(T + W[p].at(t, b8)), half[p]);
     }
 #pragma unroll
     for (u32 p = 0; p < HR_PTS; p++) {
@@ -312,7 +281,7 @@ __global__ void __launch_bounds__(HR_THREADS, 1) halton_rows_kernel(HPlanDev P)
             if (g < b) {
                 const u64 y = Y[t * b + hmod(D.fd_M, b, g * mul[t])];
                 bool exact;
-                const u64 F = hr_fixed(y, &exact);
+                const u64 F = dsum::fixed_term(y, HR_UNIT, &exact);
                 T[t * b + g] = t >= t1 ? F | (exact ? 0u : 1u) : y;
             }
         }

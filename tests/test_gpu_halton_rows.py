@@ -103,3 +103,17 @@ def test_batch_and_graph():
     first = [x.clone() for x in outs]
     _both(plan, outs)
     assert all(torch.equal(a, x) for a, x in zip(first, outs))
+
+
+def test_largest_digits():
+    # point 0 has the largest digit everywhere: sums that round up to 1 in power-of-two bases
+    import torch
+    from qmctoolscl_gb300 import halton
+    n, bases = 800000, [2, 4, 16, 256, 8, 32, 64, 128, 512, 1024, 2, 3, 5, 7, 31, 541] * 2
+    rng = np.random.Generator(np.random.SFC64(10))
+    dims = _dims(rng, 1, n - 1, bases, False, False, True)
+    for q in dims:
+        q["shifts"].fill_(q["b"] - 1)
+    x = torch.empty((1, n, len(bases)), dtype=torch.float64, device="cuda")
+    _both(halton.HaltonPlan(1, n, 0, dims, x), [x])
+    assert float(x[0, 0, 0]) == 1.0
