@@ -80,6 +80,68 @@ __global__ void __launch_bounds__(GEN_THREADS) dnb2_gen_kernel(GenArgs a)
 // ---------------------------------------------------------------------------
 // elementwise kernels
 
+// The digital shift and the float conversion over each randomisation's n*d words as one run, two words
+// (16 bytes) at a time whatever d is: a block of 32 threads over a row's columns leaves a third of them
+// idle at d = 21.  SHIFT: word w of the run takes the shift of column w mod d (staged twice
+// over in shared memory, so that a pair may wrap); a thread steps its column by a fixed amount.
+constexpr u32 RUN_VECS = 4;         // pairs in flight per thread
+constexpr u32 RUN_MAX_D = 2048;     // columns of the staged shifts
+
+template <bool SHIFT>
+__global__ void __launch_bounds__(256) dnb2_run_kernel(u64 r, u64 words, u32 d, u64 r_x, const u64 *per_l, const u64 *in,
+                                                       const u64 *shiftsb, u64 *out)
+{
+    extern __shared__ u64 sh[];
+    const u64 step = (u64)gridDim.x * 256;  // pairs between a thread's steps
+    const u32 col_step = SHIFT ? (u32)(2 * step % d) : 0u;
+    for (u64 l = blockIdx.y; l < r; l += gridDim.y) {
+        const u64 *src = in + (SHIFT ? l % r_x : l) * words;
+        u64 *dst = out + l * words;
+        const u32 ls = SHIFT ? (u32)(per_l[l % r_x] & 63) : 0u;
+        const int e = SHIFT ? 0 : (int)(u32)(0ull - per_l[l]);
+        if (SHIFT) {
+            __syncthreads();
+            for (u32 c = threadIdx.x; c <= d; c += 256) sh[c] = shiftsb[l * d + (c == d ? 0 : c)];
+            __syncthreads();
+        }
+        auto one = [&](u64 w, u64 s) {
+            return SHIFT ? (w << ls) ^ s : (u64)__double_as_longlong(to_float_bits(w, e));
+        };
+        const u32 head = (u32)(((uintptr_t)dst >> 3) & 1u);
+        if ((((uintptr_t)src >> 3) & 1u) != head) {  // never both on a 16-byte boundary: word by word
+            u32 col = SHIFT ? (u32)(((u64)blockIdx.x * 256 + threadIdx.x) % d) : 0u;
+            const u32 cs = SHIFT ? (u32)(step % d) : 0u;
+            for (u64 w = (u64)blockIdx.x * 256 + threadIdx.x; w < words; w += step) {
+                __stcs(dst + w, one(__ldcs(src + w), SHIFT ? sh[col] : 0));
+                if (SHIFT) col = col + cs >= d ? col + cs - d : col + cs;
+            }
+            continue;
+        }
+        const u64 pairs = (words - head) / 2;
+        const ulonglong2 *s2 = (const ulonglong2 *)(src + head);
+        ulonglong2 *d2 = (ulonglong2 *)(dst + head);
+        u64 q = (u64)blockIdx.x * 256 + threadIdx.x;
+        u32 col = SHIFT ? (u32)((head + 2 * q) % d) : 0u;
+        for (; q < pairs; q += RUN_VECS * step) {
+            ulonglong2 w[RUN_VECS];
+#pragma unroll
+            for (u32 u = 0; u < RUN_VECS; u++)
+                if (q + u * step < pairs) w[u] = __ldcs(s2 + q + u * step);
+#pragma unroll
+            for (u32 u = 0; u < RUN_VECS; u++) {
+                if (q + u * step < pairs)
+                    __stcs(d2 + q + u * step,
+                           make_ulonglong2(one(w[u].x, SHIFT ? sh[col] : 0), one(w[u].y, SHIFT ? sh[col + 1] : 0)));
+                if (SHIFT) col = col + col_step >= d ? col + col_step - d : col + col_step;
+            }
+        }
+        if (blockIdx.x == 0 && threadIdx.x == 0) {  // the word before the first pair and the one after the last
+            if (head && words) dst[0] = one(src[0], SHIFT ? sh[0] : 0);
+            if ((words - head) & 1) dst[words - 1] = one(src[words - 1], SHIFT ? sh[d - 1] : 0);
+        }
+    }
+}
+
 // Rows per thread per iteration: all loads of a group are issued before any
 // arithmetic so each thread keeps several loads outstanding.
 constexpr int ROWS_IN_FLIGHT = 4;
@@ -247,6 +309,28 @@ Shape rows_shape(u64 r, u64 n, u64 ngroups)
     return s;
 }
 
+// Rows of pairs (vec2) that fill their block's threads keep the row kernels, which read each column's
+// shift once; others go as runs.  us, rows / runs, (r, n, d): shift (8, 100003, 21) 56.7 / 44.0,
+// (1, 20000, 127) 14.2 / 7.0, (8, 100003, 32) 62.4 / 65.8, (1, 1000, 5) 2.1 / 2.7; float 65.6 / 43.6,
+// 12.7 / 7.0, 63.5 / 64.9, 1.9 / 2.1.
+bool as_run(u64 words, u64 d, bool vec2)
+{
+    if (words < (1ull << 17)) return false;  // a launch's latency either way, and no table to stage
+    if (!vec2) return true;
+    const u64 groups = d / 2;
+    return groups < 32 ? (groups & (groups - 1)) != 0 : groups % 32 != 0;
+}
+
+// blocks over a randomisation's run of `words`, so that all blocks are resident at once
+dim3 run_grid(u64 r, u64 words)
+{
+    const u64 y = r < 65535 ? r : 65535;
+    u64 per_l = (u64)qmcgb::sm_count() * 8 / y;
+    const u64 most = (words + 2 * 256 - 1) / (2 * 256);
+    if (per_l > most) per_l = most;
+    return dim3((unsigned)(per_l ? per_l : 1), (unsigned)y, 1);
+}
+
 unsigned flat_grid(u64 total) { return qmcgb::grid_for(total, 256, (unsigned)qmcgb::sm_count() * 32); }
 
 bool aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0; }
@@ -381,6 +465,11 @@ int qmc_dnb2_digital_shift(uint64_t r, uint64_t n, uint64_t d, uint64_t r_x, con
     if (r == 0 || n == 0 || d == 0) return QMC_OK;
     QMC_REQUIRE(r_x > 0 && lshifts && xb && shiftsb && xrb, "bad r_x or null array pointer");
     const bool vec2 = d % 2 == 0 && aligned16(xb) && aligned16(xrb);
+    if (d < RUN_MAX_D && as_run(r * n * d, d, vec2)) {
+        dnb2_run_kernel<true><<<run_grid(r, n * d), 256, (d + 1) * sizeof(u64), QMC_STREAM(s)>>>(
+            r, n * d, (u32)d, r_x, (const u64 *)lshifts, (const u64 *)xb, (const u64 *)shiftsb, (u64 *)xrb);
+        return qmcgb::launch_status("dnb2_digital_shift");
+    }
     const Shape sh = rows_shape(r, n, vec2 ? d / 2 : d);
     if (vec2)
         dnb2_shift_kernel<2><<<sh.grid, sh.block, 0, QMC_STREAM(s)>>>(r, n, d, r_x, (const u64 *)lshifts,
@@ -399,6 +488,11 @@ int qmc_dnb2_integer_to_float(uint64_t r, uint64_t n, uint64_t d, const uint64_t
     if (r == 0 || n == 0 || d == 0) return QMC_OK;
     QMC_REQUIRE(tmaxes && xb && x, "null array pointer");
     const bool vec2 = d % 2 == 0 && aligned16(xb) && aligned16(x);
+    if (as_run(r * n * d, d, vec2)) {
+        dnb2_run_kernel<false><<<run_grid(r, n * d), 256, 0, QMC_STREAM(s)>>>(
+            r, n * d, 1u, 1, (const u64 *)tmaxes, (const u64 *)xb, nullptr, (u64 *)x);
+        return qmcgb::launch_status("dnb2_integer_to_float");
+    }
     const Shape sh = rows_shape(r, n, vec2 ? d / 2 : d);
     if (vec2)
         dnb2_to_float_kernel<2><<<sh.grid, sh.block, 0, QMC_STREAM(s)>>>(r, n, d, (const u64 *)tmaxes,
