@@ -13,8 +13,8 @@
 // plan can be relaunched or replayed from a graph with no host work.
 //
 // Digital-net plans first run one matrix-preparation kernel over all
-// requests (linear matrix scrambling and interlacing, one thread per output
-// column word) into plan scratch, then the generation kernel.
+// requests (linear matrix scrambling and interlacing, one warp per matrix
+// of an output dimension) into plan scratch, then the generation kernel.
 //
 // Reference chains reproduced, bit for bit: see qmc_net_request /
 // qmc_lat_request in include/qmcgb.h.
@@ -37,8 +37,8 @@ constexpr int THREADS = 256;
 struct PrepDesc {
     u64 r, d, d_pre, mmax, alpha, nbits, tmax_alpha, r_C;
     const u64 *C, *S;
-    u64 *out;        // r*d*mmax prepared matrices
-    u64 word_begin;  // first global output word of this request
+    u64 *out;       // r*d*mmax prepared matrices
+    u64 row_begin;  // first of the request's r*d (randomisation, dimension) pairs
 };
 
 struct NetDesc {
@@ -87,38 +87,66 @@ __device__ __forceinline__ u64 lms_word(const u64 *srow, u64 col, u64 tmax_new)
 
 constexpr int MAX_ALPHA = 16;
 
-// Word loc of one request's prepared matrices: LMS of the alpha source
-// columns (dnb2_linear_matrix_scramble.c:32-48), then interlacing.
-__device__ __forceinline__ void prep_word(const PrepDesc &P, u64 loc)
+__device__ __forceinline__ u32 parity(u64 v) { return __popc((u32)v ^ (u32)(v >> 32)) & 1; }
+
+// The prepared matrix of pair `row` (randomisation l, interlaced dimension ja) of one request, by one
+// warp: LMS of the alpha source columns (dnb2_linear_matrix_scramble.c:32-48), then interlacing
+// (dnb2_interlace.c:33-41 with tmax = nbits).  Lane t holds rows t and t + 32 of the scrambling matrix and
+// takes one bit of each word per column; lane k then holds words k and k + 32 and interlaces them.
+// (A thread per word read the matrix row by row, one load after another: 36 us for 48 uneven
+// requests of 3.4 thousand pairs, 21 now, bound by the ALU.)
+__device__ __forceinline__ void prep_row(const PrepDesc &P, u64 row)
 {
-    {
-        const u64 k = loc % P.mmax, ja = (loc / P.mmax) % P.d, l = loc / (P.mmax * P.d);
-        const u64 *Cl = P.C + (l % P.r_C) * P.d_pre * P.mmax;
-        u64 words[MAX_ALPHA];
-        for (u64 a = 0; a < P.alpha; a++) {
-            const u64 j = ja * P.alpha + a;
-            const u64 col = Cl[j * P.mmax + k];
-            words[a] = P.S ? lms_word(P.S + (l * P.d_pre + j) * P.nbits, col, P.nbits) : col;
-        }
-        u64 out;
-        if (P.alpha == 1) {
-            out = words[0];
-        } else {  // dnb2_interlace.c:33-41 with tmax = nbits
-            out = 0;
-            for (u64 ta = 0; ta < P.tmax_alpha; ta++) {
-                const u64 t = ta / P.alpha;
-                if (shr64(words[ta % P.alpha], P.nbits - t - 1) & 1) out += shl64(1ull, P.tmax_alpha - ta - 1);
+    const u32 lane = threadIdx.x % 32, mmax = (u32)P.mmax;
+    const u64 l = row / P.d, ja = row % P.d;
+    const u64 *Cl = P.C + (l % P.r_C) * P.d_pre * P.mmax;
+    const u32 nbits = (u32)P.nbits;
+    u64 out[2] = {0, 0};
+    for (u64 a = 0; a < P.alpha; a++) {
+        const u64 j = ja * P.alpha + a;
+        u64 w[2];  // this lane's words of source dimension j
+#pragma unroll
+        for (u32 h = 0; h < 2; h++) w[h] = lane + 32 * h < mmax ? Cl[j * P.mmax + lane + 32 * h] : 0;
+        if (P.S) {
+            const u64 *S = P.S + (l * P.d_pre + j) * P.nbits;
+            if (P.nbits <= 64) {
+                const u64 s0 = lane < nbits ? S[lane] : 0, s1 = lane + 32 < nbits ? S[lane + 32] : 0;
+                const u64 col[2] = {w[0], w[1]};
+#pragma unroll
+                for (u32 h = 0; h < 2; h++)
+                    for (u32 k = 0; k < 32 && k + 32 * h < mmax; k++) {
+                        const u64 cv = __shfl_sync(0xFFFFFFFFu, col[h], k);
+                        const u32 p0 = __ballot_sync(0xFFFFFFFFu, parity(s0 & cv));
+                        const u32 p1 = nbits > 32 ? __ballot_sync(0xFFFFFFFFu, parity(s1 & cv)) : 0;
+                        // bit t of (p1 : p0) is digit t: bit nbits - 1 - t of the word
+                        if (lane == k) w[h] = nbits ? __brevll(((u64)p1 << 32) | p0) >> (64 - nbits) : 0;
+                    }
+            } else {
+                for (u32 h = 0; h < 2; h++)
+                    if (lane + 32 * h < mmax) w[h] = lms_word(S, w[h], P.nbits);
             }
         }
-        P.out[loc] = out;
+        if (P.alpha == 1) {
+            out[0] = w[0];
+            out[1] = w[1];
+            break;
+        }
+        u32 from = nbits - 1, to = (u32)P.tmax_alpha - 1 - (u32)a;  // shift counts are taken modulo 64
+        for (u64 ta = a; ta < P.tmax_alpha; ta += P.alpha, from--, to -= (u32)P.alpha) {
+            out[0] += shl64(shr64(w[0], from) & 1, to);
+            if (mmax > 32) out[1] += shl64(shr64(w[1], from) & 1, to);
+        }
     }
+#pragma unroll
+    for (u32 h = 0; h < 2; h++)
+        if (lane + 32 * h < mmax) P.out[row * P.mmax + lane + 32 * h] = out[h];
 }
 
-__global__ void net_prep_kernel(const PrepDesc *ps, int np, u64 total)
+__global__ void __launch_bounds__(256) net_prep_kernel(const PrepDesc *ps, int np, u64 total)
 {
-    for (u64 w = (u64)blockIdx.x * blockDim.x + threadIdx.x; w < total; w += (u64)gridDim.x * blockDim.x) {
-        const PrepDesc &P = ps[find_desc(ps, np, w, [](const PrepDesc &p) { return p.word_begin; })];
-        prep_word(P, w - P.word_begin);
+    for (u64 w = (u64)blockIdx.x * 8 + threadIdx.x / 32; w < total; w += (u64)gridDim.x * 8) {
+        const PrepDesc &P = ps[find_desc(ps, np, w, [](const PrepDesc &p) { return p.row_begin; })];
+        prep_row(P, w - P.row_begin);
     }
 }
 
@@ -264,11 +292,11 @@ struct qmc_plan {
     void *d_desc = nullptr, *d_prep = nullptr;
     u64 *d_scratch = nullptr;
     BatchCtrl *d_ctrl = nullptr;
-    u64 total_tiles = 0, prep_words = 0, coords = 0, bytes_out = 0;
+    u64 total_tiles = 0, prep_rows = 0, coords = 0, bytes_out = 0;
     size_t smem = 0;
     int ctas_per_sm = 4;
-    u32 chunk = 4;
-    u64 tile_coords = 1ull << 16;
+    u32 chunk = 1;
+    u64 tile_coords = 0;  // 0: from the plan's size (default_tile)
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
 };
@@ -283,10 +311,26 @@ void drop_graph(qmc_plan *p)
     p->graph = nullptr;
 }
 
+// Coordinates per tile where the caller has not set them: half a dozen tiles per resident CTA, so that
+// the last ones to finish cost little, between 2^15 (a net tile builds a table first) and 2^18.  48 uneven
+// net requests of 111 M coordinates: 2^14 232 us, 2^15 204, 2^16 209, 2^17 259; four tiles of 2^16
+// per grab, 238; three requests of 32768 coordinates 33 -> 15.  Lattice tiles stop at 2^16: rows of more
+// than 32 column pairs are written in several sweeps over the tile, and a tile that leaves L2 between them
+// costs (20 uneven requests up to d = 98: 2^18 3048 us, 2^16 2439).
+u64 default_tile(const qmc_plan *p)
+{
+    const u64 want = p->coords / ((u64)qmcgb::sm_count() * (u64)p->ctas_per_sm * 6);
+    const u64 most = p->kind == 1 ? 1ull << 18 : 1ull << 16;
+    u64 tile = 1ull << 15;
+    while (tile < most && 2 * tile <= want) tile *= 2;
+    return tile;
+}
+
 // Cut every request into tiles of about tile_coords coordinates and upload
 // the descriptors.
 int layout_tiles(qmc_plan *p)
 {
+    if (!p->tile_coords) p->tile_coords = default_tile(p);
     u64 tile = 0;
     if (p->kind == 1) {
         for (auto &R : p->net) {
@@ -328,9 +372,9 @@ int alloc_common(qmc_plan *p, size_t desc_bytes)
 int launch(qmc_plan *p, cudaStream_t s)
 {
     const int sms = qmcgb::sm_count();
-    if (p->kind == 1 && p->prep_words) {
-        net_prep_kernel<<<qmcgb::grid_for(p->prep_words, 256, (unsigned)sms * 8), 256, 0, s>>>(
-            (const PrepDesc *)p->d_prep, (int)p->prep.size(), p->prep_words);
+    if (p->kind == 1 && p->prep_rows) {
+        net_prep_kernel<<<qmcgb::grid_for(p->prep_rows, 8, (unsigned)sms * 8), 256, 0, s>>>(
+            (const PrepDesc *)p->d_prep, (int)p->prep.size(), p->prep_rows);
         if (int rc = qmcgb::launch_status("net_prep_kernel")) return rc;
     }
     if (p->total_tiles == 0) return QMC_OK;
@@ -413,14 +457,14 @@ int qmc_net_plan_create(const qmc_net_request *reqs, int nreq, qmc_plan **plan)
             P.r_C = Q.r_C;
             P.C = (const u64 *)Q.C;
             P.S = (const u64 *)Q.S;
-            P.word_begin = p->prep_words;
+            P.row_begin = p->prep_rows;
             P.out = (u64 *)(uintptr_t)(scratch_words);  // offset; made a pointer below
             p->prep.push_back(P);
             R.C = (const u64 *)(uintptr_t)(scratch_words);
             R.r_C = Q.r;
             R.pad = 1;  // C is an offset into plan scratch
             scratch_words += Q.r * Q.d * Q.mmax;
-            p->prep_words += Q.r * Q.d * Q.mmax;
+            p->prep_rows += Q.r * Q.d;
         } else {
             R.C = (const u64 *)Q.C;
             R.r_C = Q.r_C;
@@ -553,7 +597,7 @@ int qmc_plan_info(const qmc_plan *p, uint64_t *tiles, uint64_t *coords, uint64_t
     if (tiles) *tiles = p->total_tiles;
     if (coords) *coords = p->coords;
     if (bytes_out) *bytes_out = p->bytes_out;
-    if (launches) *launches = (p->prep_words ? 1 : 0) + (p->total_tiles ? 1 : 0);
+    if (launches) *launches = (p->prep_rows ? 1 : 0) + (p->total_tiles ? 1 : 0);
     return QMC_OK;
 }
 
@@ -622,10 +666,9 @@ int noalloc_scratch(u64 **out)
     return QMC_OK;
 }
 
-__global__ void net_prep_one_kernel(PrepDesc P, u64 total)
+__global__ void __launch_bounds__(256) net_prep_one_kernel(PrepDesc P, u64 total)
 {
-    for (u64 w = (u64)blockIdx.x * blockDim.x + threadIdx.x; w < total; w += (u64)gridDim.x * blockDim.x)
-        prep_word(P, w);
+    for (u64 w = (u64)blockIdx.x * 8 + threadIdx.x / 32; w < total; w += (u64)gridDim.x * 8) prep_row(P, w);
 }
 
 }  // namespace
@@ -655,7 +698,6 @@ extern "C" int qmc_net_gen_noalloc(const qmc_net_request *req, qmc_stream_t s)
                 "mmax=%llu), above the %d this entry point holds; use a plan (qmc_net_plan_create) for it",
                 (unsigned long long)Q.r, (unsigned long long)Q.d, (unsigned long long)Q.mmax,
                 QMC_NOALLOC_MATRIX_WORDS);
-    const u64 words = Q.r * Q.d * Q.mmax;
     cudaStream_t st = QMC_STREAM(s);
     const u64 *C = (const u64 *)Q.C;
     u64 r_C = Q.r_C;
@@ -674,7 +716,7 @@ extern "C" int qmc_net_gen_noalloc(const qmc_net_request *req, qmc_stream_t s)
         P.C = (const u64 *)Q.C;
         P.S = (const u64 *)Q.S;
         P.out = scratch;
-        net_prep_one_kernel<<<qmcgb::grid_for(words, 256, (unsigned)qmcgb::sm_count() * 8), 256, 0, st>>>(P, words);
+        net_prep_one_kernel<<<qmcgb::grid_for(Q.r * Q.d, 8, (unsigned)qmcgb::sm_count() * 8), 256, 0, st>>>(P, Q.r * Q.d);
         if (int rc = qmcgb::launch_status("net_prep_one_kernel")) return rc;
         C = scratch;
         r_C = Q.r;
