@@ -3,6 +3,7 @@
 The library is the only compute path: if it is missing or cannot be loaded,
 every call raises.  There is no CPU fallback.
 """
+import contextlib
 import ctypes
 import os
 import threading
@@ -56,6 +57,8 @@ class LibraryMissing(RuntimeError):
 def lib():
     """Load libqmcgb.so once; raise if it is not built."""
     global _lib
+    if _lib is not None:
+        return _lib
     with _lock:
         if _lib is not None:
             return _lib
@@ -103,6 +106,19 @@ def device_attributes():
     a, b, c = INT(), INT(), INT()
     check(lib().qmc_device_attributes(ctypes.byref(a), ctypes.byref(b), ctypes.byref(c)), "device_attributes")
     return {"pageable_access": a.value, "uses_host_page_tables": b.value, "sms": c.value}
+
+
+_HERE = contextlib.nullcontext()
+
+
+def on_stream(torch, stream):
+    """torch.cuda.stream(stream), or nothing where that stream and its device are the current ones
+    already: entering and leaving it cost 9 us, half of a small call."""
+    dev = getattr(stream, "device_index", None)
+    if dev is not None and torch.cuda.current_device() == dev and \
+            torch._C._cuda_getCurrentRawStream(dev) == stream.cuda_stream:
+        return _HERE
+    return torch.cuda.stream(stream)
 
 
 def writable(a):

@@ -116,6 +116,8 @@ def _parse_kwargs(kwargs):
 
 
 def _scalar(v, pos):
+    if type(v) is int or type(v) is np.uint64:
+        return int(v) & 0xFFFFFFFFFFFFFFFF
     if isinstance(v, (bool, np.bool_)) or isinstance(v, (float, np.floating)) or not hasattr(v, "__index__"):
         raise ctypes.ArgumentError("argument %d: TypeError: wrong type" % (pos + 1))
     return int(v) & 0xFFFFFFFFFFFFFFFF  # c_uint64 wraps like this
@@ -150,11 +152,8 @@ def _check_tensor(a, kind, pos, need, name):
         raise ValueError("%s has %d elements, the call needs %d" % (name, a.numel(), need))
 
 
-def _device_of(arrays, kwargs):
+def _default_device(kwargs):
     torch = _t()
-    for a in arrays:
-        if _is_torch(a):
-            return a.device
     if "device" in kwargs:
         return torch.device(kwargs["device"])
     if not torch.cuda.is_available():
@@ -172,69 +171,85 @@ def _call(name, args, kwargs):
     # host-side checks first, in the order the reference meets them: ctypes
     # argument conversion, then the preprocess hook, then array sizes
     scalars, arrays = {}, {}
+    dev, any_host = None, False
     for pos, ((an, kind), a) in enumerate(zip(spec, args)):
         if kind == "u64":
             scalars[an] = _scalar(a, pos)
         else:
-            if not _is_torch(a):
+            on_dev = _is_torch(a)
+            if not on_dev:
                 _check_numpy(a, kind, pos)
-            arrays[an] = (pos, kind, a)
+                any_host = True
+            elif dev is None:
+                dev = a.device
+            arrays[an] = (pos, kind, a, on_dev)
     pre = _PREPROCESS.get(name)
     if pre is not None:
         pre(scalars)
     need = NEED[name](scalars)
-    for an, (pos, kind, a) in arrays.items():
-        if not _is_torch(a) and a.size < need[an]:
-            raise ValueError("%s has %d elements, the call needs %d" % (an, a.size, need[an]))
+    if any_host:
+        for an, (pos, kind, a, on_dev) in arrays.items():
+            if not on_dev and a.size < need[an]:
+                raise ValueError("%s has %d elements, the call needs %d" % (an, a.size, need[an]))
     lib = _ffi.lib()  # raises if the library is not built
     torch = _t()
-    for an, (pos, kind, a) in arrays.items():
-        if _is_torch(a):
+    for an, (pos, kind, a, on_dev) in arrays.items():
+        if on_dev:
             _check_tensor(a, kind, pos, need[an], an)
-    dev = _device_of([a for (_p, _k, a) in arrays.values()], kwargs)
+    if dev is None:
+        dev = _default_device(kwargs)
+    wait = kwargs.get("wait", True)
     stream = kwargs.get("stream")
+    if stream is not None and not hasattr(stream, "cuda_stream"):
+        stream = torch.cuda.ExternalStream(int(stream), device=dev)
+    cur = torch.cuda.current_device()
+    if dev.index == cur and (stream is None or (getattr(stream, "device_index", None) == cur and stream.cuda_stream ==
+                                                torch._C._cuda_getCurrentRawStream(cur))):
+        # the device and the stream are the current ones: nothing to enter (12 us of 39 in a small call)
+        handle = torch._C._cuda_getCurrentRawStream(cur)
+        return _launch(lib, name, spec, outs, scalars, arrays, need, dev, handle, wait, any_host, t0_perf, t0_proc)
     if stream is None:
         stream = torch.cuda.current_stream(dev)
-    elif not hasattr(stream, "cuda_stream"):
-        stream = torch.cuda.ExternalStream(int(stream), device=dev)
-    handle = stream.cuda_stream
-    wait = kwargs.get("wait", True)
+    with torch.cuda.device(dev), torch.cuda.stream(stream):
+        return _launch(lib, name, spec, outs, scalars, arrays, need, dev, stream.cuda_stream, wait, any_host, t0_perf,
+                       t0_proc)
+
+
+def _launch(lib, name, spec, outs, scalars, arrays, need, dev, handle, wait, any_host, t0_perf, t0_proc):
+    torch = _t()
     in_place = IN_PLACE.get(name, set())
     host_out = []  # (numpy flat view, device tensor)
     keep = []
     ptrs = {}
-    any_host = False
-    with torch.cuda.device(dev), torch.cuda.stream(stream):
-        for an, (pos, kind, a) in arrays.items():
-            cnt = need[an]
-            if _is_torch(a):
-                ptrs[an] = a.data_ptr()
-                continue
-            any_host = True
-            tdt = torch.int64 if kind == "u64*" else torch.float64
-            flat = a.reshape(-1)[:cnt]
-            if an in outs and an not in in_place:
-                dbuf = torch.empty(max(cnt, 1), dtype=tdt, device=dev)
-            else:
-                src = flat.view(np.int64) if kind == "u64*" else flat
-                if not src.flags["WRITEABLE"]:
-                    src = src.copy()
-                dbuf = torch.from_numpy(src).to(dev) if cnt else torch.empty(1, dtype=tdt, device=dev)
-            keep.append(dbuf)
-            ptrs[an] = dbuf.data_ptr()
-            if an in outs and cnt:
-                host_out.append((flat, dbuf[:cnt]))
-        cargs = [scalars[an] if kind == "u64" else ptrs[an] for an, kind in spec]
-        fn = getattr(lib, "qmc_" + name)
-        _ffi.check(fn(*cargs, handle), name)
-        for flat, dbuf in host_out:
-            dst = torch.from_numpy(flat.view(np.int64) if flat.dtype == np.uint64 else flat)
-            dst.copy_(dbuf)
-        if any_host or wait:
-            _ffi.check(lib.qmc_device_error_check(handle), name)
-            t_proc = time.process_time() - t0_proc
+    for an, (pos, kind, a, on_dev) in arrays.items():
+        if on_dev:
+            ptrs[an] = a.data_ptr()
+            continue
+        cnt = need[an]
+        tdt = torch.int64 if kind == "u64*" else torch.float64
+        flat = a.reshape(-1)[:cnt]
+        if an in outs and an not in in_place:
+            dbuf = torch.empty(max(cnt, 1), dtype=tdt, device=dev)
         else:
-            t_proc = -1.0
+            src = flat.view(np.int64) if kind == "u64*" else flat
+            if not src.flags["WRITEABLE"]:
+                src = src.copy()
+            dbuf = torch.from_numpy(src).to(dev) if cnt else torch.empty(1, dtype=tdt, device=dev)
+        keep.append(dbuf)
+        ptrs[an] = dbuf.data_ptr()
+        if an in outs and cnt:
+            host_out.append((flat, dbuf[:cnt]))
+    cargs = [scalars[an] if kind == "u64" else ptrs[an] for an, kind in spec]
+    fn = getattr(lib, "qmc_" + name)
+    _ffi.check(fn(*cargs, handle), name)
+    for flat, dbuf in host_out:
+        dst = torch.from_numpy(flat.view(np.int64) if flat.dtype == np.uint64 else flat)
+        dst.copy_(dbuf)
+    if any_host or wait:
+        _ffi.check(lib.qmc_device_error_check(handle), name)
+        t_proc = time.process_time() - t0_proc
+    else:
+        t_proc = -1.0
     return time.perf_counter() - t0_perf, t_proc
 
 

@@ -29,12 +29,29 @@ class _Args:
     def __init__(self, stream=None, device=None, direct_out=True):
         torch = _t()
         self.torch = torch
-        self.dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
-        self.stream = torch.cuda.current_stream(self.dev) if stream is None else stream
+        cur = torch.cuda.current_device()
+        self.dev = torch.device("cuda", cur) if device is None else torch.device(device)
+        if stream is None and self.dev.index == cur:  # the stream object is made when it is asked for
+            self._stream, self._parts = None, torch._C._cuda_getCurrentStream(cur)
+            self.handle = torch._C._cuda_getCurrentRawStream(cur)
+        else:
+            self._stream = torch.cuda.current_stream(self.dev) if stream is None else stream
+            self.handle = self._stream.cuda_stream
         self.keep, self.back = [], []
         self.h2d_bytes = self.d2h_bytes = 0
         self.direct_out = direct_out
         self.direct = False
+
+    @property
+    def stream(self):
+        if self._stream is None:
+            sid, index, kind = self._parts
+            self._stream = self.torch.cuda.Stream(stream_id=sid, device_index=index, device_type=kind)
+        return self._stream
+
+    def scope(self):
+        """The call's stream made the current one, for the copies of host arrays."""
+        return _ffi._HERE if self._stream is None else _ffi.on_stream(self.torch, self._stream)
 
     def ptr(self, a, dtype, count, out=False, name="array"):
         torch = self.torch
@@ -93,12 +110,12 @@ def lattice_gen_shift(r, n, d, n_start, g, shifts, xr, order="gray", stream=None
     if order not in ("gray", "natural"):
         raise ValueError("order must be 'gray' or 'natural'")
     A = _Args(stream, direct_out=direct_out)
-    with torch.cuda.stream(A.stream):
+    with A.scope():
         pg = A.ptr(g, np.uint64, r * d, name="g")
         ps = A.ptr(shifts, np.float64, r * d, name="shifts")
         px = A.ptr(xr, np.float64, r * n * d, out=True, name="xr")
         rc = _ffi.lib().qmc_lat_gen_shift(r, n, d, n_start, 1 if order == "gray" else 0, pg, ps, px,
-                                          A.stream.cuda_stream)
+                                          A.handle)
         _ffi.check(rc, "lattice_gen_shift")
         A.finish()
     return A
@@ -124,7 +141,7 @@ def dnb2_gen_fused(r, n, d, n_start, mmax, C, r_C=None, order="natural", lshifts
     r_C = r if r_C is None else int(r_C)
     r_x = r if r_x is None else int(r_x)
     A = _Args(stream)
-    with torch.cuda.stream(A.stream):
+    with A.scope():
         pC = A.ptr(C, np.uint64, r_C * d * mmax, name="C")
         pl = A.ptr(lshifts, np.uint64, r_x, name="lshifts")
         ps = A.ptr(shiftsb, np.uint64, r * d, name="shiftsb")
@@ -132,7 +149,7 @@ def dnb2_gen_fused(r, n, d, n_start, mmax, C, r_C=None, order="natural", lshifts
         pxb = A.ptr(xrb, np.uint64, r * n * d, out=True, name="xrb")
         px = A.ptr(x, np.float64, r * n * d, out=True, name="x")
         rc = _ffi.lib().qmc_dnb2_gen_fused(r, n, d, n_start, mmax, pC, r_C, 1 if order == "gray" else 0, pl, r_x,
-                                           ps, pt, pxb, px, A.stream.cuda_stream)
+                                           ps, pt, pxb, px, A.handle)
         _ffi.check(rc, "dnb2_gen_fused")
         A.finish()
     return A

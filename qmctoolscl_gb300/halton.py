@@ -227,7 +227,7 @@ def generalized_net_fused(r, n, n_start, dims, x, check=True, stream=None):
     torch = _torch()
     r, n, n_start = int(r), int(n), int(n_start)
     A = _Args(stream)
-    with torch.cuda.stream(A.stream):
+    with A.scope():
         structs = []
         for j, q in enumerate(dims):
             b, tmax, mmax = int(q["b"]), int(q["tmax"]), int(q["mmax"])

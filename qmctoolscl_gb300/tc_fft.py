@@ -23,7 +23,7 @@ def _run(fn_name, d1, d2, n_half, arrays, stream=None):
     d1, d2, n_half = int(d1), int(d2), int(n_half)
     count = d1 * d2 * 2 * n_half
     s = stream if stream is not None else torch.cuda.current_stream()
-    with torch.cuda.stream(s):  # the copies in on the call's stream, ahead of the kernels
+    with _ffi.on_stream(torch, s):  # the copies in on the call's stream, ahead of the kernels
         devs, back = _device_arrays(torch, arrays, count)
         rc = getattr(_ffi.lib(), fn_name)(d1, d2, n_half, *[t.data_ptr() for t in devs], s.cuda_stream)
         _ffi.check(rc, fn_name)
@@ -85,7 +85,7 @@ def _fused(fn_name, d1, d2, n_half, lams, data, divide, scale, stream, twiddles=
     n = 2 * n_half
     count = d1 * d2 * n
     s = stream if stream is not None else torch.cuda.current_stream()
-    with torch.cuda.stream(s):  # every copy in on the call's stream, ahead of the kernels
+    with _ffi.on_stream(torch, s):  # every copy in on the call's stream, ahead of the kernels
         lam, per_element = _lam_tensors(torch, lams, n, count)
         devs, back = _device_arrays(torch, data, count)
         tw = [torch.empty(n, dtype=torch.float64, device="cuda") for _ in range(2)] if twiddles else []
