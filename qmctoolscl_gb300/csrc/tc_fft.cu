@@ -269,6 +269,23 @@ __global__ void tc_stepB_kernel()
     }
 }
 
+// eight columns of the accumulators (two for real data, else three), added in FP32
+template <bool REAL>
+__device__ __forceinline__ void read_sum(u32 acc, float (&y)[8])
+{
+    u32 v0[8], v1[8], v2[8];
+    tc::tmem_ld8(acc, v0);
+    if (!REAL) tc::tmem_ld8(acc + 32, v1);
+    tc::tmem_ld8(acc + 64, v2);
+    tc::tmem_wait_ld();
+#pragma unroll
+    for (u32 m = 0; m < 8; m++) {
+        y[m] = __uint_as_float(v0[m]);
+        if (!REAL) y[m] += __uint_as_float(v1[m]);
+        y[m] += __uint_as_float(v2[m]);
+    }
+}
+
 template <int KIND>
 __global__ void __launch_bounds__(FT_THREADS, 3) tc_pass_kernel(TcPassArgs a, unsigned *err)
 {
@@ -281,7 +298,7 @@ __global__ void __launch_bounds__(FT_THREADS, 3) tc_pass_kernel(TcPassArgs a, un
     __shared__ __align__(8) u64 bar;
     __shared__ u32 tmem_base;
     constexpr bool REAL = KIND == TC_WHT || KIND == TC_WCONV;
-    const u32 warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const u32 warp = threadIdx.x / 32;
     const u32 NOUT = REAL ? 16u : 32u;      // GEMM N
     const u32 KIN = REAL ? 16u : 32u;       // reals per group and split
 
@@ -397,6 +414,18 @@ __global__ void __launch_bounds__(FT_THREADS, 3) tc_pass_kernel(TcPassArgs a, un
         }
         __syncthreads();
         prefetch_tile(tile + gridDim.x);
+        // y <- y * lam * lam_scale or y / lam * lam_scale
+        auto pointwise = [&](float &yr, float &yi, float lr, float lm) {
+            const float xr = yr, xi = yi;
+            if (a.divide) {
+                const float q = __fdiv_rn(a.lam_scale, fmaf(lr, lr, lm * lm));
+                yr = (xr * lr + xi * lm) * q;
+                yi = (xi * lr - xr * lm) * q;
+            } else {
+                yr = (xr * lr - xi * lm) * a.lam_scale;
+                yi = (xr * lm + xi * lr) * a.lam_scale;
+            }
+        };
         // the steps over the pass's bits for step kind SK (FFT, IFFT or WHT): false when a wait ran out
         auto steps = [&](auto skc) -> bool {
             constexpr int SK = decltype(skc)::value;
@@ -529,69 +558,75 @@ __global__ void __launch_bounds__(FT_THREADS, 3) tc_pass_kernel(TcPassArgs a, un
                         }
                         tc::mma_commit(&bar);
                     }
+                    // the fused pass: lam at the outputs of the last step, loaded while the MMAs run
+                    float lamr[8], lami[8];
+                    if (KIND == TC_CONV && SK == TC_FFT && st + 1 == n16 + nrem) {
+                        const u32 gi = 128 * mt + (threadIdx.x & 127), half = threadIdx.x >> 7;
+                        const u32 cc = gi & ctm, qq = gi >> ctl;
+                        const u32 q0 = (qq & ((1u << lo) - 1)) | ((qq >> lo) << (lo + 4));
+                        const u64 f = base + ((u64)(q0 + (half * 8u << lo)) << a.k0) + cc;
+                        const u64 at = a.lam_all ? f : (f & ((1ull << a.L) - 1)), step = 1ull << k;
+                        u64 b[8];
+#pragma unroll
+                        for (u32 m = 0; m < 8; m++) b[m] = f < a.total ? ((const u64 *)a.lr)[at + m * step] : 0;
+#pragma unroll
+                        for (u32 m = 0; m < 8; m++) lamr[m] = to_f32_on(b[m], m & 1u);
+#pragma unroll
+                        for (u32 m = 0; m < 8; m++) b[m] = f < a.total ? ((const u64 *)a.li)[at + m * step] : 0;
+#pragma unroll
+                        for (u32 m = 0; m < 8; m++) lami[m] = to_f32_on(b[m], m & 1u);
+                    }
                     ok = __syncthreads_and(tc::mbar_wait(&bar, phase, WAIT_LIMIT) ? 1 : 0);
                     phase ^= 1;
                     tc::fence_after_sync();
                     if (!ok) break;
-                    // read back: warps 0-3 the real outputs, warps 4-7 the imaginary ones
+                    // read back: a thread takes the outputs half*8 .. +7 of its group, both components, and
+                    // for the inverse step their post-twiddle w^-br(q), or in the fused pass lam, before it
+                    // writes them.  (As sweeps over shared memory of their own, with a barrier each, and a
+                    // component per thread here: 64 vectors of 2^20, inverse 1393 us, 1260 now, product
+                    // 2759 and 2336; 100 of 2^16, product 311 and 262.)
                     {
-                        const u32 gi = 128 * mt + 32 * (warp & 3) + lane;
-                        const u32 cc = gi & ctm, qq = gi >> ctl;
-                        const u32 qlo = qq & ((1u << lo) - 1), qhi = qq >> lo;
-                        const u32 S = (1u << lo) * ct;
-                        const u32 e0 = (qlo | (qhi << (lo + 4))) * ct + cc;
-                        const u32 col0 = (SK == TC_WHT) ? 0u : 16u * (warp >> 2);
-                        if (SK != TC_WHT || warp < 4) {
-                            const u32 lanes = (32 * (warp & 3)) << 16;
-                            u32 v0[16], v1[16], v2[16];
-                            tc::tmem_ld16(tmem + lanes + col0, v0);
-                            if (SK != TC_WHT) tc::tmem_ld16(tmem + lanes + 32 + col0, v1);
-                            tc::tmem_ld16(tmem + lanes + 64 + col0, v2);
-                            tc::tmem_wait_ld();
-                            float *dst = (SK == TC_WHT || warp < 4) ? sr : si;
-#pragma unroll
-                            for (u32 m = 0; m < 16; m++) {
-                                float y = __uint_as_float(v0[m]);
-                                if (SK != TC_WHT) y += __uint_as_float(v1[m]);
-                                y += __uint_as_float(v2[m]);
-                                dst[slot(e0 + m * S)] = y;
-                            }
-                        }
-                    }
-                    // the next M-tile's operand build reads only its own groups' elements, and its
-                    // MMAs (which overwrite the accumulators read here) start after the barrier that
-                    // follows the build: only the last M-tile of a step, and the inverse step's
-                    // post-twiddle (other threads' outputs), need a barrier here
-                    if (SK == TC_IFFT || mt + 1 == FT_GROUPS / 128) {
-                        tc::fence_before_sync();
-                        __syncthreads();
-                    }
-                    if (SK == TC_IFFT) {
-                        // post-twiddle w^-br(q) of the inverse step
                         const u32 gi = 128 * mt + (threadIdx.x & 127), half = threadIdx.x >> 7;
                         const u32 cc = gi & ctm, qq = gi >> ctl;
                         const u32 qlo = qq & ((1u << lo) - 1), qhi = qq >> lo;
                         const u32 S = (1u << lo) * ct;
                         const u32 e0 = (qlo | (qhi << (lo + 4))) * ct + cc + half * 8 * S;
-                        const u32 cgrp = ((u32)base + (qlo << a.k0) + cc) & ((1u << k) - 1);
-                        const u32 cg = cgrp << (28 - k);
-                        if (k > 0) {
-                            const HalfTwiddles tw = half_twiddles(tab, cg, half, k + 4, 1.0f);  // as in the forward step
+                        const u32 acc = tmem + ((32 * (warp & 3)) << 16) + half * 8;
+                        float yr[8], yi[8];
+                        read_sum<REAL>(acc, yr);
+                        if (SK != TC_WHT) read_sum<REAL>(acc + 16, yi);
+                        if (SK == TC_IFFT && k > 0) {
+                            const u32 cgrp = ((u32)base + (qlo << a.k0) + cc) & ((1u << k) - 1);
+                            const HalfTwiddles tw = half_twiddles(tab, cgrp << (28 - k), half, k + 4, 1.0f);
 #pragma unroll
-                            for (u32 pp = 0; pp < 8; pp += 2) {
+                            for (u32 pp = 0; pp < 8; pp += 2) {  // as in the forward step
                                 const u32 jj = ((pp >> 1) & 1u) * 2u + ((pp >> 2) & 1u);  // brev3(pp)
                                 float pwr[2], pwi[2];
                                 pair_twiddles(tw, jj, pwr[0], pwi[0], pwr[1], pwi[1]);
 #pragma unroll
                                 for (u32 h = 0; h < 2; h++) {
-                                    const u32 e = slot(e0 + (pp + h) * S);
-                                    const float wr = pwr[h], wi = pwi[h];
-                                    const float xr_ = sr[e], xi_ = si[e];
-                                    sr[e] = xr_ * wr - xi_ * wi;
-                                    si[e] = xr_ * wi + xi_ * wr;
+                                    const float xr_ = yr[pp + h], xi_ = yi[pp + h];
+                                    yr[pp + h] = xr_ * pwr[h] - xi_ * pwi[h];
+                                    yi[pp + h] = xr_ * pwi[h] + xi_ * pwr[h];
                                 }
                             }
                         }
+                        if (KIND == TC_CONV && SK == TC_FFT && st + 1 == n16 + nrem) {
+#pragma unroll
+                            for (u32 m = 0; m < 8; m++) pointwise(yr[m], yi[m], lamr[m], lami[m]);
+                        }
+#pragma unroll
+                        for (u32 m = 0; m < 8; m++) {
+                            const u32 e = slot(e0 + m * S);
+                            sr[e] = yr[m];
+                            if (SK != TC_WHT) si[e] = yi[m];
+                        }
+                    }
+                    // the next M-tile's operand build reads only its own groups' elements, and its
+                    // MMAs (which overwrite the accumulators read here) start after the barrier that
+                    // follows the build: only the last M-tile of a step needs a barrier here
+                    if (mt + 1 == FT_GROUPS / 128) {
+                        tc::fence_before_sync();
                         __syncthreads();
                     }
                 }
@@ -602,23 +637,14 @@ __global__ void __launch_bounds__(FT_THREADS, 3) tc_pass_kernel(TcPassArgs a, un
         if constexpr (KIND == TC_CONV) {
             ok = steps(std::integral_constant<int, TC_FFT>{});
             if (ok) {
-                // y <- y * lam * s or y / lam * s at the forward transform's output positions f
-                for (u32 e = threadIdx.x; e < Q * ct; e += FT_THREADS) {
+                // after radix-2 steps the pointwise operation is a sweep of its own, at output positions f
+                for (u32 e = threadIdx.x; e < Q * ct && (a.k1 - a.k0) % 4; e += FT_THREADS) {
                     const u64 f = base + ((u64)(e >> ctl) << a.k0) + (e & ctm);
                     if (f >= a.total) continue;
                     const u64 li_ = a.lam_all ? f : (f & ((1ull << a.L) - 1));
                     const float lr = to_f32((u64)__double_as_longlong(a.lr[li_]));
                     const float lm = to_f32((u64)__double_as_longlong(a.li[li_]));
-                    const u32 sl = slot(e);
-                    const float yr = sr[sl], yi = si[sl];
-                    if (a.divide) {
-                        const float q = __fdiv_rn(a.lam_scale, fmaf(lr, lr, lm * lm));
-                        sr[sl] = (yr * lr + yi * lm) * q;
-                        si[sl] = (yi * lr - yr * lm) * q;
-                    } else {
-                        sr[sl] = (yr * lr - yi * lm) * a.lam_scale;
-                        si[sl] = (yr * lm + yi * lr) * a.lam_scale;
-                    }
+                    pointwise(sr[slot(e)], si[slot(e)], lr, lm);
                 }
                 // operand B: the inverse step matrix for the inverse steps, then the forward one again
                 for (u32 i = threadIdx.x; i < FT_B_WORDS; i += FT_THREADS) ((uint4 *)sB)[i] = g_stepB[1][i];

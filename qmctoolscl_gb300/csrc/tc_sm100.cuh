@@ -139,6 +139,15 @@ __device__ __forceinline__ void tmem_ld16(u32 taddr, u32 (&r)[16])
         : "memory");
 }
 
+// the same for columns col..col+7
+__device__ __forceinline__ void tmem_ld8(u32 taddr, u32 (&r)[8])
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
+}
+
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // byte offset of element (row, k) in a K-major no-swizzle operand tile with
