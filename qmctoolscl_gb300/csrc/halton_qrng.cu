@@ -8,17 +8,18 @@
 // (halton_qrng.c:133-140).  res is d x n, dimension-major.
 //
 // Bit for bit with less work.  The value after the steps k = 31 .. k0 depends on i / b^k0 alone, so
-// consecutive points share it: a CTA takes a dimension and 4096 consecutive points, computes the
-// values of the top level (the first k0 with at most 256 of them) each by its own chain, then
-// every level below from the one above with one step per value, and the points with one step
+// consecutive points share it: a warp takes a run of consecutive points of a dimension, computes the
+// values of the top level (the first k0 with at most 32 of them) each by its own chain, a lane each,
+// then every level below from the one above with one step per value, and the points with one step
 // each: b / (b - 1) steps a point instead of its digit count.  Steps above an index's digits
-// add the digit shifts only and are the same for every point (P[m]).
+// add the digit shifts only and are the same for every point (P[m]).  The run is what a warp's
+// share of the CTA's points and its level arrays hold (340 b points); warps wait for no other after the
+// tables (levels shared by a CTA, with barriers between them: 0.69 ms, a third of it at the barriers).
 //
 // A step RN(RN(v + c) / b) takes four FP64 operations (qrng_step_fp64), or integer arithmetic
-// (qrng_step.cuh); of the last level, the one with all the points, every warp takes QRNG_INT_WARPS of
-// eight rounds in the integer form, so that the narrow FP64 unit and the integer pipes both work
-// (FP64 70 %, ALU 55 % busy: what bounds it, with the barriers between the levels).
-// n = 2^20, d = 100: 2.51 ms with the whole chains (a quarter of them by FP64 divides), 0.69 ms now.
+// (qrng_step.cuh); of the last level, the one with all the points, four rounds of eight take the
+// integer form, so that the narrow FP64 unit and the integer pipes both work: what bounds it.
+// n = 2^20, d = 100: 2.51 ms with the whole chains (a quarter of them by FP64 divides), 0.60 ms now.
 #include <algorithm>
 
 #include "common.cuh"
@@ -90,20 +91,24 @@ __constant__ int c_qrng_mult[QRNG_DIMS] = {
 };
 
 constexpr u32 QRNG_THREADS = 256;
-constexpr u32 QRNG_CHUNK = 4096;      // points of a step of a CTA (2048: 713 us, 1024: 810, against 689)
+constexpr u32 QRNG_CTAS = 4;        // per SM (n = 2^20, d = 100: 5 with fewer registers 652 us against 618)
+constexpr u32 QRNG_WAVES = 4;       // waves of CTAs: 3: 612 us, 4: 603, 5: 602, 8: 618, 16: 706
+constexpr u32 QRNG_LEVEL = 340;     // values of a warp's largest level: 200: 607 us, 340: 603, 500 (3 CTAs): 637
+constexpr u32 QRNG_POINTS = 4096;   // a CTA's least, but for calls of less than a wave
 constexpr u32 QRNG_MAX_B = 2424;
-constexpr u32 QRNG_INT_WARPS = 4;     // 0: 980 us, 2: 812, 3: 734, 4: 712, 5: 803 (n = 2^20, d = 100)
+constexpr u32 QRNG_INT_ROUNDS = 4;  // of eight: 3: 635 us, 4: 618, 5: 725 (the rounds of a CTA in common)
 
 struct QrngTables {
-    double level[2][QRNG_CHUNK / 2 + 2];  // the values of a level: odd levels in [1]
-    double c0[QRNG_MAX_B];                // the last step's addend by digit
-    double P[33];                         // prefix after the steps k = 31 .. m with digits 0
-    u32 s[32];                            // digit shifts
+    double odd[QRNG_THREADS / 32][QRNG_LEVEL + 2];       // a warp's values of a level, by the level's parity
+    double even[QRNG_THREADS / 32][QRNG_LEVEL / 2 + 2];
+    u32 c0[QRNG_MAX_B];  // the last step's addend by digit: a double's upper word, the lower is 0
+    double P[33];        // prefix after the steps k = 31 .. m with digits 0
+    u32 s[32];           // digit shifts
 };
 
-__global__ void __launch_bounds__(QRNG_THREADS, 4) halton_qrng_kernel(int n, int n0, int generalized, double *res,
-                                                                   const double *randu, const int *dvec,
-                                                                   unsigned *err)
+__global__ void __launch_bounds__(QRNG_THREADS, QRNG_CTAS) halton_qrng_kernel(int n, int n0, u64 per, int generalized,
+                                                                           double *res, const double *randu,
+                                                                           const int *dvec, unsigned *err)
 {
     extern __shared__ __align__(16) unsigned char sm[];
     QrngTables &S = *(QrngTables *)sm;
@@ -124,68 +129,73 @@ __global__ void __launch_bounds__(QRNG_THREADS, 4) halton_qrng_kernel(int n, int
         double u = 0.0;
         S.P[32] = u;
         for (int k = 31; k >= 0; k--) {
-            u = __ddiv_rn(__dadd_rn(u, (double)S.s[k]), bd);
+            const u32 c = S.s[k];
+            u = c < b ? qrng_step_fp64(u, (double)c, bd, rb) : __ddiv_rn(__dadd_rn(u, (double)c), bd);
             S.P[k] = u;
         }
     }
     // halton_qrng.c:135: the digit's addend
     auto addend = [&](u32 digit, u32 k) { return fd_mod(fb, f * digit + S.s[k]); };
-    for (u32 g = tid; g < b; g += QRNG_THREADS) S.c0[g] = (double)addend(g, 0);
+    for (u32 g = tid; g < b; g += QRNG_THREADS) S.c0[g] = (u32)__double2hiint((double)addend(g, 0));
     __syncthreads();
     double *out = res + (u64)j * (u64)n;
-    const u64 per = ((u64)n + gridDim.x - 1) / gridDim.x, q_end = min((u64)n, (blockIdx.x + 1) * per);
-    for (u64 q = blockIdx.x * per; q < q_end;) {
-        const u32 t0 = (u32)(int)((long long)n0 + (long long)q);  // halton_qrng.c:110: tmp = i
-        const u32 cnt = (u32)min(min(q_end - q, (u64)QRNG_CHUNK), (1ull << 32) - t0);  // a negative n0 wraps to 0
-        const u32 t1 = t0 + (cnt - 1);
-        // the top level
-        u32 K = 1, first = fd_div(fb, t0), last = fd_div(fb, t1);
-        while (last - first >= QRNG_THREADS) {
-            K++;
-            first = fd_div(fb, first);
-            last = fd_div(fb, last);
-        }
-        if (tid <= last - first) {
-            u32 dig[32], m = K;
-            for (u32 h = first + tid; h; m++) {
-                const u32 up = fd_div(fb, h);
-                dig[m & 31u] = h - up * b;
-                h = up;
+    const u64 q_end = min((u64)n, (blockIdx.x + 1) * per);
+    const u32 warp = tid / 32, lane = tid % 32;
+    double *odd = S.odd[warp], *even = S.even[warp];
+    const u64 span = min((u64)(QRNG_LEVEL * b / 32 * 32), (per + QRNG_THREADS - 1) / QRNG_THREADS * 32);
+    for (u64 q0 = blockIdx.x * per + warp * span; q0 < q_end; q0 += span * (QRNG_THREADS / 32)) {
+        const u64 q1 = min(q_end, q0 + span);
+        for (u64 q = q0; q < q1;) {
+            const u32 t0 = (u32)(int)((long long)n0 + (long long)q);    // halton_qrng.c:110: tmp = i
+            const u32 cnt = (u32)min(q1 - q, (1ull << 32) - t0);  // a negative n0 wraps to 0
+            // the top level, a value per lane
+            u32 K = 1, first = fd_div(fb, t0), last = fd_div(fb, t0 + (cnt - 1));
+            while (last - first >= 32) {
+                K++;
+                first = fd_div(fb, first);
+                last = fd_div(fb, last);
             }
-            double v = S.P[m];
-            while (m-- > K) v = qrng_step_fp64(v, (double)addend(dig[m & 31u], m), bd, rb);
-            S.level[K & 1][tid] = v;
-        }
-        // the levels below it
-        for (u32 k = K - 1; k >= 1; k--) {
-            __syncthreads();
-            const u32 parent0 = first;
-            u32 lo = t0, hi = t1;
-            for (u32 i = 0; i < k; i++) {
-                lo = fd_div(fb, lo);
-                hi = fd_div(fb, hi);
+            __syncwarp();  // the values of the run before have been read
+            if (lane <= last - first) {
+                u32 dig[32], m = K;
+                for (u32 h = first + lane; h; m++) {
+                    const u32 up = fd_div(fb, h);
+                    dig[m & 31u] = h - up * b;
+                    h = up;
+                }
+                double v = S.P[m];
+                while (m-- > K) v = qrng_step_fp64(v, (double)addend(dig[m & 31u], m), bd, rb);
+                (K & 1u ? odd : even)[lane] = v;
             }
-            for (u32 e = tid; e <= hi - lo; e += QRNG_THREADS) {
-                const u32 h = lo + e, up = fd_div(fb, h);
-                S.level[k & 1][e] =
-                    qrng_step_fp64(S.level[(k + 1) & 1][up - parent0], (double)addend(h - up * b, k), bd, rb);
+            // the levels below it
+            for (u32 k = K - 1; k >= 1; k--) {
+                u32 lo = t0, hi = t0 + (cnt - 1);
+                for (u32 i = 0; i < k; i++) {
+                    lo = fd_div(fb, lo);
+                    hi = fd_div(fb, hi);
+                }
+                const double *level = k & 1u ? even : odd;
+                double *dst = k & 1u ? odd : even;
+                __syncwarp();
+                for (u32 e = lane; e <= hi - lo; e += 32) {
+                    const u32 h = lo + e, up = fd_div(fb, h);
+                    dst[e] = qrng_step_fp64(level[up - first], (double)addend(h - up * b, k), bd, rb);
+                }
+                first = lo;
             }
-            first = lo;
+            __syncwarp();
+            // the points
+            for (u32 e = lane, i = warp; e < cnt; e += 32, i += 3) {
+                const u32 t = t0 + e, up = fd_div(fb, t), digit = t - up * b;
+                const double v = odd[up - first];
+                u64 o;
+                if ((i & 7u) < QRNG_INT_ROUNDS && qstep::step(as_bits(v), addend(digit, 0), qd, o))
+                    out[q + e] = as_double(o);
+                else
+                    out[q + e] = qrng_step_fp64(v, __hiloint2double((int)S.c0[digit], 0), bd, rb);
+            }
+            q += cnt;
         }
-        __syncthreads();
-        // the points
-        for (u32 e = tid; e < cnt; e += QRNG_THREADS) {
-            const u32 t = t0 + e, up = fd_div(fb, t), digit = t - up * b;
-            const bool integer = ((e / QRNG_THREADS * 3 + tid / 32) & 7u) < QRNG_INT_WARPS;
-            const double v = S.level[1][up - first], c = S.c0[digit];
-            u64 o;
-            if (integer && qstep::step(as_bits(v), addend(digit, 0), qd, o))
-                out[q + e] = as_double(o);
-            else
-                out[q + e] = qrng_step_fp64(v, c, bd, rb);
-        }
-        __syncthreads();
-        q += cnt;
     }
 }
 
@@ -204,16 +214,17 @@ int qmc_halton_qrng(int n, int d, int n0, int generalized, double *res, const do
     QMC_REQUIRE(res && randu_d_32 && dvec, "halton_qrng: null array pointer");
     unsigned *err = qmcgb::device_error_ptr();
     QMC_REQUIRE(err, "device error word unavailable");
-    // about eight waves of CTAs (four per SM) over all dimensions; a CTA builds its dimension's tables
-    // first, so it takes at least 1024 points (what is left of a chunk costs as much as the whole)
-    const u64 waves = (u64)qmcgb::sm_count() * 4 * 8;
+    // CTAs of all dimensions in a few waves; a CTA builds its dimension's tables first, so it takes at
+    // least QRNG_POINTS points, or 1024 where that leaves SMs idle
+    const u64 waves = (u64)qmcgb::sm_count() * QRNG_CTAS * QRNG_WAVES;
     u64 per_dim = std::max<u64>(1, waves / (u64)d);
-    per_dim = std::max<u64>(std::min<u64>(per_dim, ((u64)n + QRNG_CHUNK - 1) / QRNG_CHUNK),
-                            std::min<u64>(((u64)n + 1023) / 1024, (u64)qmcgb::sm_count() * 4 / (u64)d));
-    const unsigned gx = (unsigned)std::max<u64>(1, per_dim);
+    per_dim = std::max<u64>(std::min<u64>(per_dim, ((u64)n + QRNG_POINTS - 1) / QRNG_POINTS),
+                            std::min<u64>(((u64)n + 1023) / 1024, (u64)qmcgb::sm_count() * QRNG_CTAS / (u64)d));
+    const u64 per = ((u64)n + std::max<u64>(1, per_dim) - 1) / std::max<u64>(1, per_dim);
+    const unsigned gx = (unsigned)(((u64)n + per - 1) / per);
     if (int rc = qmcgb::raise_smem_limit((const void *)halton_qrng_kernel, sizeof(QrngTables), "halton_qrng")) return rc;
     halton_qrng_kernel<<<dim3(gx, (unsigned)d, 1), QRNG_THREADS, sizeof(QrngTables), QMC_STREAM(s)>>>(
-        n, n0, generalized, res, randu_d_32, dvec, err);
+        n, n0, per, generalized, res, randu_d_32, dvec, err);
     return qmcgb::launch_status("halton_qrng");
 }
 
