@@ -46,7 +46,7 @@
 // four digits is below half an ulp of v the lane stops.  The tile of doubles
 // is staged in shared memory and stored as contiguous rows.  The grid holds
 // exactly the CTAs resident at once, striding over the equal-cost tiles.
-// Plans of 24 million coordinates and more whose tables fit shared memory generate with
+// Plans of a few million coordinates and more whose tables fit shared memory generate with
 // halton_rows_kernel (halton_rows.cuh) instead: first 100 primes, r=32, n=2^18, 20.3 -> 8.0 ms,
 // issue-bound (66 % of the issue slots, ALU 52 %, FP64 34 %) where this kernel waits for the FP64 unit.
 #include <algorithm>
@@ -634,7 +634,7 @@ void plan_rows(qmc_halton_plan *p, std::vector<HGroup> &groups)
 {
     const u64 sms = (u64)qmcgb::sm_count();
     auto up = [](size_t v) { return (v + 15) & ~(size_t)15; };
-    const u32 nt = HR_THREADS, max_per = 16;
+    const u32 nt = HR_THREADS;
     size_t smem = 0;
     double work = 0, coords = 0;
     std::vector<double> cost;
@@ -648,7 +648,7 @@ void plan_rows(qmc_halton_plan *p, std::vector<HGroup> &groups)
             double c = 0;
             while (j < R.d && G.nd < HR_DIMS && (G.nd == 0 || j % HR_DIMS)) {
                 const HDim &h = p->hd[R.dim0 + j];
-                const size_t pitch = 2 * (h.tmax | 1u), hs = up(((32 * max_per - 1) / h.bK2 + 2) * pitch);
+                const size_t pitch = 2 * (h.tmax | 1u), hs = up(((32 * HR_RUN - 1) / h.bK2 + 2) * pitch);
                 const size_t T = up((size_t)h.tmax * h.b * 8), L = up(h.bK2 * pitch), H = hs * (nt / 32),
                              C = up((size_t)h.mmax * h.tmax * 4);
                 if (used + T + L + H + C > HR_MAX_SMEM) break;
@@ -670,7 +670,7 @@ void plan_rows(qmc_halton_plan *p, std::vector<HGroup> &groups)
             coords += (double)(R.r * R.n) * G.nd;
         }
     }
-    // The tables of a CTA cost about as much as two of its steps: it keeps them for up to 16 while
+    // The tables of a CTA cost about as much as two of its steps: it keeps them for up to HR_STEPS while
     // there are a dozen CTAs of equal work per SM, heaviest (smallest bases) first.  Plans below
     // HR_MIN_COORDS coordinates, or with fewer than HR_MIN_POINTS points per randomisation on
     // average, finish sooner on the warp kernel, which has no tables to set up.
@@ -686,7 +686,7 @@ void plan_rows(qmc_halton_plan *p, std::vector<HGroup> &groups)
     for (size_t g = 0; g < groups.size(); g++) {
         HGroup &G = groups[g];
         const HReq &R = p->hreq[G.req];
-        G.span = nt * std::max<u64>(HR_PTS, std::min<u64>(max_per, (u64)(target / cost[g])));
+        G.span = nt * std::max<u64>(HR_PTS, std::min<u64>(HR_STEPS, (u64)(target / cost[g])));
         G.splits = (u32)((R.n + G.span - 1) / G.span);
         G.item0 = item0;
         item0 += R.r * G.splits;

@@ -25,9 +25,15 @@
 // entry has no inverse, and K > 1 (b < 32), read the low part from a table L[x][t].
 //
 // A CTA owns up to four consecutive dimensions of one randomisation (32 bytes of each output
-// row, one store) and a range of points, a run of it per warp: no barrier after the tables, so
+// row, one store) and a range of points, in sections of a run per warp: no barrier after the tables, so
 // that a warp with a point to redo holds up no other (with steps in common the barriers were
-// two thirds of the time).
+// two thirds of the time).  The term tables serve all sections of the CTA, the sums H one.
+//
+// What bounds it: issue (73 % of the slots), the shared-memory pipe (79 %: a table read is two
+// wavefronts, a 32-byte piece of 32 rows up to 32) and the ALU (58 %).  First 100 primes, r = 32, n = 2^18: 6.85 ms
+// (all FP64 adds 20.3; one section per CTA, and registers spilled for what the redone points need, 8.07).  The
+// stores alone, a CTA after another in a column of 32 bytes, take 4.4 ms; with the CTAs of a row next
+// to each other 2.6, but the whole no less (6.99: its CTAs differ in length).
 #pragma once
 
 namespace {
@@ -36,15 +42,18 @@ constexpr u32 HR_DIMS = 4;
 constexpr u32 HR_PTS = 2;          // points of a lane: 32 apart
 constexpr u32 HR_THREADS = 1024;   // 64 registers: 8.0 ms; 768 threads 8.8, 4 points on 640 threads 9.0 (first 100
                                    // primes, r=32, n=2^18; 4 dimensions unrolled 8.9: instruction cache)
+constexpr u32 HR_RUN = 16;         // most times 32 points in a warp's run (8: 7.21 ms, 16: 6.85, 32: 6.77, more memory)
+constexpr u32 HR_STEPS = 64;       // most times HR_THREADS points of a CTA (16: 7.86 ms, 64: 6.92, 128: 7.02)
 constexpr u32 HR_TINY = 9;         // integer rows need v >= 2^-(HR_TINY + 1)
 constexpr int HR_UNIT = 79;        // F counts 2^-79: the integer rows' terms sum to 2^63 at most
 constexpr u32 HR_HEAD_BITS = 16;   // b^t1 >= 2^16
-// Below these the warp kernel, which has no tables to set up, finishes sooner.  us, warp kernel / this
-// one, (r, n, d): (16, 8192, 100) 336 / 502, (32, 16384, 20) 487 / 744, (8, 65536, 37) 672 / 720,
-// (1, 262144, 100) 657 / 586, (4, 262144, 100) 2578 / 1162, (32, 262144, 100) 20320 / 8070, 64 uneven requests
-// of 73 M coordinates 2991 / 1536.
-constexpr double HR_MIN_COORDS = 2.4e7, HR_MIN_POINTS = 16000;
-constexpr u32 HR_MAX_SMEM = 216 * 1024;  // and 7 KB of HConst
+// Below these the warp kernel, which has no tables to set up, finishes sooner.  us of preparation and run,
+// warp kernel / this one, (r, n, d): (1, 20000, 20) 90 / 154, (4, 16384, 10) 121 / 157, (2, 30000, 50) 177 / 169,
+// (16, 8192, 20) 197 / 181, (1, 10^6, 3) 647 / 339; of the run: (300, 1024, 100) 768 / 1386, (256, 2048, 100)
+// 1267 / 1560, (32, 4096, 50) 211 / 185, (128, 4096, 100) 1266 / 979, (32, 262144, 100) 20320 / 6850, 64 uneven
+// requests of 73 M coordinates 3027 / 1489.
+constexpr double HR_MIN_COORDS = 2.4e6, HR_MIN_POINTS = 4000;
+constexpr u32 HR_MAX_SMEM = 216 * 1024;  // and 6 KB of HConst, HSlow and output rows
 
 // Up to four dimensions and the byte offsets of their tables in shared memory.
 struct HGroup {
@@ -151,6 +160,13 @@ struct HConst {
     u32 T, H, L, h0;  // addresses of the tables; H, h0: this warp's and its first hi
 };
 
+// What the plain chain of a point needs of a dimension, in shared memory.
+struct HSlow {
+    const HDim *D;
+    const u64 *Y;
+    const u32 *mul;
+};
+
 // The digits of one point: byte offsets in the rows of the term table.  LOW: the low part from
 // the table row at `lp`, else the thread's own x8.
 template <bool LOW>
@@ -165,8 +181,11 @@ struct HDigits {
 
 // The plain FP64 chain of one point, terms from the plan's table (mul: the rows' multipliers).
 template <bool LOW>
-__device__ __noinline__ double hr_point(const HDigits<LOW> W, const HDim &D, const u64 *Y, const u32 *mul)
+__device__ __noinline__ double hr_point(const HDigits<LOW> W, const HSlow *slow)
 {
+    const HDim &D = *slow->D;
+    const u64 *Y = slow->Y;
+    const u32 *mul = slow->mul;
     const u32 b = D.b, tmax = D.tmax;
     const u64 M = D.fd_M;
     double v = 0.0;
@@ -207,7 +226,7 @@ __device__ __forceinline__ void hr_values(const HDigits<LOW> (&W)[HR_PTS], u32 T
 #pragma unroll
         for (u32 p = 0; p < HR_PTS; p++) acc[p] = dsum::add_even(acc[p], hr_ld64(T + W[p].at(t, b8)), half[p]);
     }
-#pragma unroll 1
+#pragma unroll 2
     for (; t < rows; t++) {
         T += b8;
 #pragma unroll
@@ -225,8 +244,8 @@ __device__ __forceinline__ void hr_values(const HDigits<LOW> (&W)[HR_PTS], u32 T
 
 // One dimension of the lane's points.
 template <bool LOW>
-__device__ __forceinline__ void hr_dim(const HConst &c, const u32 (&index)[HR_PTS],
-                                       const HDim &D, const u64 *Y, const u32 *mul, double (&v)[HR_PTS])
+__device__ __forceinline__ void hr_dim(const HConst &c, const u32 (&index)[HR_PTS], const HSlow *slow,
+                                       double (&v)[HR_PTS])
 {
     HDigits<LOW> W[HR_PTS];
     bool ok[HR_PTS];
@@ -239,13 +258,15 @@ __device__ __forceinline__ void hr_dim(const HConst &c, const u32 (&index)[HR_PT
     hr_values<LOW>(W, c.T, c.b8, c.info, v, ok);
 #pragma unroll
     for (u32 p = 0; p < HR_PTS; p++)
-        if (!ok[p]) v[p] = hr_point<LOW>(W[p], D, Y, mul);
+        if (!ok[p]) v[p] = hr_point<LOW>(W[p], slow);
 }
 
 __global__ void __launch_bounds__(HR_THREADS, 1) halton_rows_kernel(HPlanDev P)
 {
     extern __shared__ __align__(16) unsigned char sm[];
     __shared__ HConst consts[32][HR_DIMS];
+    __shared__ HSlow slow[HR_DIMS];
+    __shared__ double *outs[32];  // a warp's output row
     const u32 tid = threadIdx.x, nt = blockDim.x, warp = tid / 32, lane = tid % 32, nw = nt / 32;
     const u64 item = blockIdx.x;
     u32 glo = 0, ghi = P.ngroups - 1;  // the group whose CTAs hold this one
@@ -285,6 +306,7 @@ __global__ void __launch_bounds__(HR_THREADS, 1) halton_rows_kernel(HPlanDev P)
                 T[t * b + g] = t >= t1 ? F | (exact ? 0u : 1u) : y;
             }
         }
+        if (tid == 0) slow[q] = HSlow{&D, Y, mul};
         u32 *Cs = (u32 *)(sm + G.c_off[q]);
         for (u32 e = tid; e < D.mmax * tmax; e += nt) Cs[e] = Cnl[D.c_off + e];
     }
@@ -306,61 +328,68 @@ __global__ void __launch_bounds__(HR_THREADS, 1) halton_rows_kernel(HPlanDev P)
                 L[x * pitch + t] = (u16)(8u * dim_mod(D, acc));
             }
     }
-    // this warp's run of the CTA's points
-    const u64 i0 = split * G.span + (u64)warp * (G.span / nw);
-    const u64 i_end = min(min(R.n, (split + 1) * G.span), i0 + G.span / nw);
-    const u32 base = (u32)(R.n_start + i0);
-    for (u32 q = 0; q < nd && i0 < i_end; q++) {
-        const HDim &D = dims[q];
-        const u32 tmax = D.tmax, pitch = tmax | 1u, h0 = hdiv(D.fdK2_M, base);
-        const u32 nh = hdiv(D.fdK2_M, base + (u32)(i_end - i0) - 1) - h0 + 1;
-        const u32 *Cs = (const u32 *)(sm + G.c_off[q]);
-        u16 *H = (u16 *)(sm + G.h_off[q] + warp * G.h_size[q]);
-        if (lane == 0)
-            hc[q] = HConst{info_l[q], 8 * D.b, D.bK2, 2 * pitch, D.fdK2_M, sa + G.t_off[q],
-                           sa + G.h_off[q] + warp * G.h_size[q], sa + G.l_off[q], h0};
-        for (u32 e = lane; e < nh * tmax; e += 32) {
-            const u32 u = e / tmax, t = e - u * tmax;
-            u32 acc = 0, h = h0 + u;
-            for (u32 k = D.K2; h && k < D.mmax; k++) {
-                const u32 d = hdiv(D.fd_M, h);
-                acc += (h - d * D.b) * Cs[k * tmax + t];
-                h = d;
-            }
-            H[u * pitch + t] = (u16)(8u * dim_mod(D, acc));
-        }
-    }
     __syncthreads();
-    const bool v4 = nd == 4 && R.d % 4 == 0 && ((uintptr_t)R.x & 31u) == 0;
-    const u64 d = R.d;
-    double *out0 = R.x + l * R.n * d + G.j0;
-    for (u64 i = i0 + lane; i < i_end; i += 32 * HR_PTS) {
-        // a point past the end repeats the first: no branch around the shared work
-        u32 index[HR_PTS];
-#pragma unroll
-        for (u32 p = 0; p < HR_PTS; p++) index[p] = base + (u32)(i + 32 * p < i_end ? i + 32 * p - i0 : i - i0);
-        double v[HR_DIMS][HR_PTS];
-#pragma unroll 1
-        for (u32 q = 0; q < HR_DIMS; q++) {
-            if (q >= nd) break;
-            const HConst c = hc[q];
-            if (c.info >> 31)
-                hr_dim<true>(c, index, dims[q], Yl + dims[q].y_off, mul_l + dims[q].s_off, v[q]);
-            else
-                hr_dim<false>(c, index, dims[q], Yl + dims[q].y_off, mul_l + dims[q].s_off, v[q]);
+    const u32 d = (u32)R.d;
+    const bool v4 = nd == 4 && d % 4 == 0 && ((uintptr_t)R.x & 31u) == 0;
+    // the CTA's points in sections, a run of each per warp: the tables above serve all of them, the
+    // sums of the high digits one
+    const u64 c0 = split * G.span, c_end = min(R.n, c0 + G.span);
+    const u32 per = (u32)(G.span / nt), sections = (per + HR_RUN - 1) / HR_RUN;
+    const u32 run = (per + sections - 1) / sections * 32;
+    for (u64 i0 = c0 + warp * run; i0 < c_end; i0 += nw * run) {
+        const u32 cnt = (u32)min((u64)run, c_end - i0);
+        const u32 base = (u32)(R.n_start + i0);
+        __syncwarp();  // the sums of the section before have been read
+        if (lane == 0) outs[warp] = R.x + (l * R.n + i0) * R.d + G.j0;
+        for (u32 q = 0; q < nd; q++) {
+            const HDim &D = dims[q];
+            const u32 tmax = D.tmax, pitch = tmax | 1u, h0 = hdiv(D.fdK2_M, base);
+            const u32 nh = hdiv(D.fdK2_M, base + cnt - 1) - h0 + 1;
+            const u32 *Cs = (const u32 *)(sm + G.c_off[q]);
+            u16 *H = (u16 *)(sm + G.h_off[q] + warp * G.h_size[q]);
+            if (lane == 0)
+                hc[q] = HConst{info_l[q], 8 * D.b, D.bK2, 2 * pitch, D.fdK2_M, sa + G.t_off[q],
+                               sa + G.h_off[q] + warp * G.h_size[q], sa + G.l_off[q], h0};
+            for (u32 e = lane; e < nh * tmax; e += 32) {
+                const u32 u = e / tmax, t = e - u * tmax;
+                u32 acc = 0, h = h0 + u;
+                for (u32 k = D.K2; h && k < D.mmax; k++) {
+                    const u32 d = hdiv(D.fd_M, h);
+                    acc += (h - d * D.b) * Cs[k * tmax + t];
+                    h = d;
+                }
+                H[u * pitch + t] = (u16)(8u * dim_mod(D, acc));
+            }
         }
+        __syncwarp();
+        for (u32 i = lane; i < cnt; i += 32 * HR_PTS) {
+            // a point past the end repeats the first: no branch around the shared work
+            u32 index[HR_PTS];
 #pragma unroll
-        for (u32 p = 0; p < HR_PTS; p++) {
-            if (i + 32 * p >= i_end) break;
-            double *out = out0 + (i + 32 * p) * d;
-            if (v4) {
-                asm volatile("st.global.cs.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(out), "d"(v[0][p]), "d"(v[1][p]),
-                             "d"(v[2][p]), "d"(v[3][p])
-                             : "memory");
-            } else {
+            for (u32 p = 0; p < HR_PTS; p++) index[p] = base + (i + 32 * p < cnt ? i + 32 * p : i);
+            double v[HR_DIMS][HR_PTS];
+#pragma unroll 1
+            for (u32 q = 0; q < HR_DIMS; q++) {
+                if (q >= nd) break;
+                const HConst c = hc[q];
+                if (c.info >> 31)
+                    hr_dim<true>(c, index, slow + q, v[q]);
+                else
+                    hr_dim<false>(c, index, slow + q, v[q]);
+            }
 #pragma unroll
-                for (u32 q = 0; q < HR_DIMS; q++)
-                    if (q < nd) __stcs(out + q, v[q][p]);
+            for (u32 p = 0; p < HR_PTS; p++) {
+                if (i + 32 * p >= cnt) break;
+                double *out = outs[warp] + (u64)(i + 32 * p) * d;
+                if (v4) {
+                    asm volatile("st.global.cs.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(out), "d"(v[0][p]), "d"(v[1][p]),
+                                 "d"(v[2][p]), "d"(v[3][p])
+                                 : "memory");
+                } else {
+#pragma unroll
+                    for (u32 q = 0; q < HR_DIMS; q++)
+                        if (q < nd) __stcs(out + q, v[q][p]);
+                }
             }
         }
     }

@@ -1,4 +1,4 @@
-"""The fused Halton plan on its shared-memory tables (plans of 24 million coordinates and more) against the
+"""The fused Halton plan on its shared-memory tables (plans of a few million coordinates and more) against the
 same plan on the warp kernel (any split of the adds selects it; that kernel is held to the oracle in
 test_gpu_halton.py), bit for bit over the whole output: primes, composite and power-of-two bases (ties in
 every row), large bases (groups of fewer dimensions), matrices without an inverse, every set of steps,
@@ -117,3 +117,26 @@ def test_largest_digits():
     x = torch.empty((1, n, len(bases)), dtype=torch.float64, device="cuda")
     _both(halton.HaltonPlan(1, n, 0, dims, x), [x])
     assert float(x[0, 0, 0]) == 1.0
+
+
+@pytest.mark.parametrize("r,n,n_start,bases", [(16, (1 << 20) + 777, 0, [2, 3, 5, 7, 29, 31, 37, 101, 541, 547]),
+                                               (40, 300001, 1 << 20, [2, 4, 6, 9, 16, 25, 36, 64, 97, 211, 256, 540])])
+def test_sections(r, n, n_start, bases):
+    """Plans of 120 million coordinates and more, where a CTA's points come in several sections: sections
+    that end early and last CTAs with part of their points."""
+    import torch
+    from qmctoolscl_gb300 import halton
+    rng = np.random.Generator(np.random.SFC64(n))
+    x = torch.empty((r, n, len(bases)), dtype=torch.float64, device="cuda")
+    _both(halton.HaltonPlan(r, n, n_start, _dims(rng, r, n_start + n - 1, bases, True, True, True), x), [x])
+
+
+@pytest.mark.parametrize("r,n,n_start,bases", [(1, 1000003, 0, [2, 3, 5]), (64, 4097, 65535, [2, 3, 7, 37, 53, 101, 541, 9, 4, 25]),
+                                               (3, 40000, 99, PRIMES[:21]), (150, 4001, 0, [31, 29, 2, 547, 64])])
+def test_smallest_plans(r, n, n_start, bases):
+    """Plans of a few million coordinates: two steps of points per CTA."""
+    import torch
+    from qmctoolscl_gb300 import halton
+    rng = np.random.Generator(np.random.SFC64(n))
+    x = torch.empty((r, n, len(bases)), dtype=torch.float64, device="cuda")
+    _both(halton.HaltonPlan(r, n, n_start, _dims(rng, r, n_start + n - 1, bases, True, True, True), x), [x])
