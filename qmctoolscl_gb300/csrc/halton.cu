@@ -640,6 +640,14 @@ void plan_rows(qmc_halton_plan *p, std::vector<HGroup> &groups)
     std::vector<double> cost;
     for (size_t q = 0; q < p->hreq.size(); q++) {
         const HReq &R = p->hreq[q];
+        // pinned host outputs: the 32-byte pieces of a row go over the CPU link one by one (r = 4, n = 2^18,
+        // d = 100: 138 GB/s, and 26 for d = 21; whole lines of the warp kernel 173 and 169)
+        cudaPointerAttributes at;
+        if (cudaPointerGetAttributes(&at, R.x) != cudaSuccess) {
+            cudaGetLastError();
+            return;
+        }
+        if (at.type != cudaMemoryTypeDevice) return;
         for (u64 j = 0; j < R.d;) {
             HGroup G{};
             G.req = (u32)q;

@@ -140,3 +140,20 @@ def test_smallest_plans(r, n, n_start, bases):
     rng = np.random.Generator(np.random.SFC64(n))
     x = torch.empty((r, n, len(bases)), dtype=torch.float64, device="cuda")
     _both(halton.HaltonPlan(r, n, n_start, _dims(rng, r, n_start + n - 1, bases, True, True, True), x), [x])
+
+
+@pytest.mark.parametrize("r,n,d", [(2, 130001, 12), (1, 262144, 21)])
+def test_pinned_output(r, n, d):
+    """Outputs in pinned host memory, which keep the warp kernel."""
+    import torch
+    from qmctoolscl_gb300 import batch, halton
+    rng = np.random.Generator(np.random.SFC64(n))
+    dims = _dims(rng, r, n - 1, PRIMES[:d], True, True, True)
+    x = torch.empty((r, n, d), dtype=torch.float64, device="cuda")
+    host = batch.pinned_empty((r, n, d))
+    for out in (x, host):
+        plan = halton.HaltonPlan(r, n, 0, dims, out)
+        plan.prepare()
+        plan.run()
+    torch.cuda.synchronize()
+    assert np.array_equal(x.cpu().numpy(), host)
