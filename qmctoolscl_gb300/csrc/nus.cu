@@ -82,8 +82,8 @@ __global__ void nus_keys_kernel(NusDims m, const u64 *__restrict__ xb, const u64
 // come first (one warp per 256 points, then a scan per generator); the stream itself, the only
 // serial part, then runs without looking at the draws; and the draws take their bits from it, a
 // thread per point.  With the draws formatted and stored inside the serial loop, a step took
-// 68 cycles; the bare chain of 64-bit integer operations takes about 30 on one warp (32
-// generators).  r=4, d=8, n=200000: 7.15 ms for the draws before, 2.99 now (stream 2.93, 28 cycles a step).
+// 68 cycles; the bare chain of 64-bit integer operations takes 24 on one warp (32
+// generators: the ALU).  r=4, d=8, n=200000: 7.15 ms for the draws before, 2.59 now (stream 2.53).
 
 constexpr u32 DT = 256;  // points per warp of the counting and formatting passes: all loads in flight at once
 
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(32) nus_draw_scan_kernel(NusDims m, const u64 
     if (lane == 0) info[g] = DrawInfo{full + half_outputs(half, has), has, (u32)st[5], 0};
 }
 
-constexpr u32 STREAM_STEPS = 32;  // outputs per generator between two barriers
+constexpr u32 STREAM_STEPS = 64;  // outputs per generator between two barriers (32: the whole call 4.80 ms, 64: 4.45)
 
 // The streams of 32 generators: warp 0, alone on its quarter of the SM, steps them (a lane each) into
 // shared memory, the other three warps write whole 256-byte row segments behind it.
@@ -198,9 +198,15 @@ __global__ void __launch_bounds__(128) nus_stream_kernel(NusDims m, u64 *__restr
     if (warp == 0 && g < m.S) r = Sfc64{st[0], st[1], st[2], st[3], 0, 0};
     for (u32 i0 = 0, k = 0; i0 < most; i0 += STREAM_STEPS, k ^= 1) {
         if (warp == 0) {
-            if (i0 + STREAM_STEPS <= least) {
+            if (i0 + STREAM_STEPS <= least && __all_sync(0xFFFFFFFFu, (u32)r.w <= 0u - STREAM_STEPS)) {
+                // the counter's upper half stands still: an instruction less of a step's thirteen on the ALU
+                const u64 high = r.w & 0xFFFFFFFF00000000ull;
+                const u32 low = (u32)r.w;
 #pragma unroll
-                for (u32 s = 0; s < STREAM_STEPS; s++) buf[k][s][lane] = r.next64();
+                for (u32 s = 0; s < STREAM_STEPS; s++) {
+                    r.w = high | (low + s);
+                    buf[k][s][lane] = r.next64();
+                }
             } else {
                 for (u32 s = 0; s < STREAM_STEPS && i0 + s < need; s++) buf[k][s][lane] = r.next64();
             }
@@ -208,14 +214,17 @@ __global__ void __launch_bounds__(128) nus_stream_kernel(NusDims m, u64 *__restr
         __syncthreads();  // also: the other warps are done with the other buffer
         if (warp != 0) {
             // all reads ahead of all stores: row by row, three warps took longer than the 32 steps
-            u64 x[11];
+#pragma unroll 1
+            for (u32 h = 0; h < STREAM_STEPS; h += 32) {
+                u64 x[11];
 #pragma unroll
-            for (u32 e = 0; e < 11; e++) x[e] = buf[k][lane][min(warp - 1 + 3 * e, 31u)];
-            u64 *row = raw + (u64)(g0 + warp - 1) * m.NP + i0 + lane;
+                for (u32 e = 0; e < 11; e++) x[e] = buf[k][h + lane][min(warp - 1 + 3 * e, 31u)];
+                u64 *row = raw + (u64)(g0 + warp - 1) * m.NP + i0 + h + lane;
 #pragma unroll
-            for (u32 e = 0; e < 11; e++) {
-                const u32 q = warp - 1 + 3 * e, end = __shfl_sync(0xFFFFFFFFu, need, q & 31u);
-                if (q < 32 && i0 + lane < end) row[(u64)(3 * e) * m.NP] = x[e];
+                for (u32 e = 0; e < 11; e++) {
+                    const u32 q = warp - 1 + 3 * e, end = __shfl_sync(0xFFFFFFFFu, need, q & 31u);
+                    if (q < 32 && i0 + h + lane < end) row[(u64)(3 * e) * m.NP] = x[e];
+                }
             }
         }
     }

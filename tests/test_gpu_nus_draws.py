@@ -29,3 +29,28 @@ def test_sparse_half_draws(share):
     close = np.arange(1, n) % (share * 300) < share
     xb[:, 1:][:, close] = xb[:, :-1][:, close] ^ np.uint64(1 << 20)
     _check_against_oracle(rng, 1, n, 2, 1, 64, 64, [xb, xb[:, ::-1].copy()])
+
+
+@pytest.mark.parametrize("n", [63, 64, 65, 127, 129, 300, 20000])
+def test_counters_near_their_upper_half(n):
+    """Streams whose 64-bit counter carries into its upper half in, before and after a block of outputs."""
+    import oracle
+    import qmctoolscl_gb300 as q
+    from .test_gpu_nus import _states
+    rng = np.random.Generator(np.random.SFC64(n))
+    d = 5
+    gens = [np.random.Generator(np.random.SFC64(k)) for k in range(d)]
+    for k, g in enumerate(gens):
+        state = g.bit_generator.state
+        state["state"]["state"][3] = np.uint64((1 << 32) * (k + 1) - (10, 64, 65, 200, 1)[k])
+        g.bit_generator.state = state
+    words = _states(gens).reshape(-1).copy()
+    xb = rng.integers(0, 1 << 63, (1, n, d), dtype=np.uint64) * np.uint64(2)
+    want, got = np.zeros((1, n, d), np.uint64), np.zeros((1, n, d), np.uint64)
+    forest = oracle.NusForest(d)
+    forest.scramble(1, n, d, 1, 64, 64, words, xb, want)
+    roots = np.array([q.NUSNode_dnb2() for _ in range(d)]).reshape(1, d)
+    q.dnb2_nested_uniform_scramble(1, n, d, 1, 64, 64, np.array(gens, dtype=object).reshape(1, d), roots, xb, got)
+    forest.close()
+    assert np.array_equal(got, want)
+    assert np.array_equal(_states(gens).reshape(-1), words)
