@@ -46,9 +46,9 @@
 // four digits is below half an ulp of v the lane stops.  The tile of doubles
 // is staged in shared memory and stored as contiguous rows.  The grid holds
 // exactly the CTAs resident at once, striding over the equal-cost tiles.
-// Plans of a few million coordinates and more whose tables fit shared memory generate with
-// halton_rows_kernel (halton_rows.cuh) instead: first 100 primes, r=32, n=2^18, 20.3 -> 8.0 ms,
-// issue-bound (66 % of the issue slots, ALU 52 %, FP64 34 %) where this kernel waits for the FP64 unit.
+// Plans of a few million coordinates and more into device memory whose tables fit shared memory generate
+// with halton_rows_kernel (halton_rows.cuh) instead: first 100 primes, r=32, n=2^18, 20.3 -> 6.85 ms, bound by
+// issue and shared memory (73 and 79 %; FP64 45 %) where this kernel waits for the FP64 unit.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -230,6 +230,8 @@ __global__ void halton_recip_kernel(HPlanDev P, u64 *recip)
 // (64-bit wrapping add), then (double)digit * recip_t as
 // gdn_integer_to_float.c:36-37.  Lane 0 records the row's largest exponent in
 // the tail table (whose words are numbered exactly like the rows).
+// FLAGS: the row flags of the table kernel too (3 of 79 us of preparation, r = 28, d = 42).
+template <bool FLAGS>
 __global__ void halton_terms_kernel(HPlanDev P, const PrepDim *pd, u64 *Y, u32 *tail, u32 *flags)
 {
     const u32 lane = threadIdx.x % 32;
@@ -245,7 +247,8 @@ __global__ void halton_terms_kernel(HPlanDev P, const PrepDim *pd, u64 *Y, u32 *
         u64 *yrow = Y + R.y_base + l * R.y_per_l + D.y_off + t * D.b;
         if (t >= D.tmax) {  // padding row: +0 terms, no tail
             for (u32 g = lane; g < D.b; g += 32) yrow[g] = 0;
-            if (lane == 0) tail[row] = flags[row] = 0;
+            if (lane == 0) tail[row] = 0;
+            if (FLAGS && lane == 0) flags[row] = 0;
             continue;
         }
         const double rc = as_double(P.recip[D.r_off + t]);
@@ -258,13 +261,13 @@ __global__ void halton_terms_kernel(HPlanDev P, const PrepDim *pd, u64 *Y, u32 *
             const u64 y = dig ? as_bits(__dmul_rn(rc, __ull2double_rn(dig))) : 0;
             yrow[g] = y;
             mx = max(mx, y);  // non-negative doubles order like their bits
-            fl |= hr_term_flags(y, dig, D.b);
+            if (FLAGS) fl |= hr_term_flags(y, dig, D.b);
         }
-        fl = __reduce_or_sync(0xffffffffu, fl);
+        if (FLAGS) fl = __reduce_or_sync(0xffffffffu, fl);
         for (int o = 16; o; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         if (lane == 0) {
             tail[row] = (u32)(mx >> 52);
-            flags[row] = fl;
+            if (FLAGS) flags[row] = fl;
         }
     }
 }
@@ -571,9 +574,14 @@ int prepare_launch(qmc_halton_plan *p, cudaStream_t st)
     if (int rc = qmcgb::launch_status("halton_lms_kernel")) return rc;
     halton_recip_kernel<<<qmcgb::grid_for(p->P.ndims, 128, 1024), 128, 0, st>>>(p->P, (u64 *)p->d_recip);
     if (int rc = qmcgb::launch_status("halton_recip_kernel")) return rc;
-    halton_terms_kernel<<<qmcgb::grid_for(p->P.rows * 32, 256, cap), 256, 0, st>>>(p->P, (const PrepDim *)p->d_prep,
-                                                                                  (u64 *)p->d_Y, (u32 *)p->d_tail,
-                                                                                  (u32 *)p->d_flags);
+    const unsigned tg = qmcgb::grid_for(p->P.rows * 32, 256, cap);
+    const PrepDim *pd = (const PrepDim *)p->d_prep;
+    u64 *Y = (u64 *)p->d_Y;
+    u32 *tail = (u32 *)p->d_tail;
+    if (p->items)
+        halton_terms_kernel<true><<<tg, 256, 0, st>>>(p->P, pd, Y, tail, (u32 *)p->d_flags);
+    else
+        halton_terms_kernel<false><<<tg, 256, 0, st>>>(p->P, pd, Y, tail, nullptr);
     if (int rc = qmcgb::launch_status("halton_terms_kernel")) return rc;
     if (p->items) {
         halton_norm_kernel<<<qmcgb::grid_for(p->P.rows, 128, cap), 128, 0, st>>>(p->P, (const u32 *)p->d_C,
