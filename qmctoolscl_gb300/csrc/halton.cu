@@ -77,10 +77,6 @@ struct HDim {
     u32 tpad;      // tmax rounded up to a multiple of HT_GROUP: term rows past tmax hold +0
     u64 fd_M;      // direct-remainder constant for b (any 32-bit x)
     u64 fdK_M;     // the same for b^K
-    // generation from shared-memory tables (halton_rows.cuh)
-    u32 t1, rows;  // FP64 rows at the front, rows that can change a sum of at least 2^-10
-    u32 K2, bK2;   // low digits of its index split, b^K2
-    u64 fdK2_M;
     u64 c_off;     // offset of this dimension's (mmax x tmax) block inside a randomisation's C block
     u64 y_off;     // offset of its (tpad x b) term rows inside a randomisation's Y block
     u64 s_off;     // offset of its tpad digits inside the request's tail blocks
@@ -104,6 +100,7 @@ struct HReq {
 };
 
 struct HGroup;
+struct HRowDim;
 
 struct HPlanDev {
     u64 nreq, total_c, rows, titems, ntiles, ndims;
@@ -116,6 +113,7 @@ struct HPlanDev {
     const u16 *order;    // per request, its dimension ids (request-relative) grouped by warp
     const u32 *wstart;   // per request, HT_WARPS + 1 offsets into its order
     const HGroup *groups;
+    const HRowDim *rdims;  // numbered like dims
     u32 ngroups;
     const u32 *Cn, *mul;  // matrices divided by their lowest digit's row, and those divisors (numbered like tail)
     const u32 *info;      // per (request, l, j): the sections of its rows
@@ -529,11 +527,12 @@ bool assign_adds(std::vector<HDim> &hd, double share)
 struct qmc_halton_plan {
     HPlanDev P{};
     std::vector<HDim> hd;
+    std::vector<HRowDim> rd;
     std::vector<HReq> hreq;
     std::vector<PrepDim> prep;
     void *d_req = nullptr, *d_dims = nullptr, *d_C = nullptr, *d_Y = nullptr, *d_recip = nullptr, *d_tail = nullptr;
     void *d_order = nullptr, *d_wstart = nullptr, *d_prep = nullptr;
-    void *d_groups = nullptr, *d_Cn = nullptr, *d_mul = nullptr, *d_flags = nullptr, *d_info = nullptr;
+    void *d_groups = nullptr, *d_rdims = nullptr, *d_Cn = nullptr, *d_mul = nullptr, *d_flags = nullptr, *d_info = nullptr;
     u64 items = 0;       // CTAs of halton_rows_kernel; 0: some table does not fit
     u32 rows_threads = 0;
     size_t rows_smem = 0;
@@ -664,8 +663,9 @@ void plan_rows(qmc_halton_plan *p, std::vector<HGroup> &groups)
             double c = 0;
             while (j < R.d && G.nd < HR_DIMS && (G.nd == 0 || j % HR_DIMS)) {
                 const HDim &h = p->hd[R.dim0 + j];
-                const size_t pitch = 2 * (h.tmax | 1u), hs = up(((32 * HR_RUN - 1) / h.bK2 + 2) * pitch);
-                const size_t T = up((size_t)h.tmax * h.b * 8), L = up(h.bK2 * pitch), H = hs * (nt / 32),
+                const HRowDim &rd = p->rd[R.dim0 + j];
+                const size_t pitch = 2 * (h.tmax | 1u), hs = up(((32 * HR_RUN - 1) / rd.bK2 + 2) * pitch);
+                const size_t T = up((size_t)h.tmax * h.b * 8), L = up(rd.bK2 * pitch), H = hs * (nt / 32),
                              C = up((size_t)h.mmax * h.tmax * 4);
                 if (used + T + L + H + C > HR_MAX_SMEM) break;
                 G.t_off[G.nd] = (u32)used;
@@ -674,7 +674,7 @@ void plan_rows(qmc_halton_plan *p, std::vector<HGroup> &groups)
                 G.c_off[G.nd] = (u32)(used + T + L + H);
                 G.h_size[G.nd] = (u32)hs;
                 used += T + L + H + C;
-                c += h.rows + 6.0;  // a step of a dimension: its rows, and about six rows' worth around them
+                c += rd.rows + 6.0;  // a step of a dimension: its rows, and about six rows' worth around them
                 G.nd++;
                 j++;
             }
@@ -806,19 +806,21 @@ int qmc_halton_batch_create(const qmc_halton_request *reqs, int nreq, qmc_halton
             // rows until b^t1 >= 2^16; rows whose terms (below b^-t) can reach half a last place of a
             // sum of 2^-10 or more: 2^-63
             const double bits = std::log2((double)h.b);
-            h.t1 = 1;
-            for (u64 v = h.b; v < (1ull << HR_HEAD_BITS) && h.t1 < h.tmax; v *= h.b) h.t1++;
-            h.rows = std::min<u32>(h.tmax, (u32)std::ceil((double)(54 + HR_TINY) / bits + 1e-9));
-            h.rows = std::max(h.rows, h.t1);
+            HRowDim rd{};
+            rd.t1 = 1;
+            for (u64 v = h.b; v < (1ull << HR_HEAD_BITS) && rd.t1 < h.tmax; v *= h.b) rd.t1++;
+            rd.rows = std::min<u32>(h.tmax, (u32)std::ceil((double)(54 + HR_TINY) / bits + 1e-9));
+            rd.rows = std::max(rd.rows, rd.t1);
             // low digits: one from b = 32 on, else as many as make a hundred values, so that a step's
             // points share few values of the rest
-            h.K2 = 1;
-            h.bK2 = h.b;
-            while (h.b < 32 && h.bK2 < 100) {
-                h.bK2 *= h.b;
-                h.K2++;
+            rd.K2 = 1;
+            rd.bK2 = h.b;
+            while (h.b < 32 && rd.bK2 < 100) {
+                rd.bK2 *= h.b;
+                rd.K2++;
             }
-            h.fdK2_M = fastdiv32_make(h.bK2).M;
+            rd.fdK2_M = fastdiv32_make(rd.bK2).M;
+            p->rd.push_back(rd);
             h.c_off = c_off;
             h.y_off = y_off;
             h.s_off = s_off;
@@ -900,10 +902,12 @@ int qmc_halton_batch_create(const qmc_halton_request *reqs, int nreq, qmc_halton
     alloc(&p->d_flags, t_base * sizeof(u32));
     if (p->items) {
         alloc(&p->d_groups, groups.size() * sizeof(HGroup));
+        alloc(&p->d_rdims, ndims * sizeof(HRowDim));
         alloc(&p->d_Cn, c_base * sizeof(u32));
         alloc(&p->d_mul, t_base * sizeof(u32));
         alloc(&p->d_info, tl_base * sizeof(u32));
         put(p->d_groups, groups.data(), groups.size() * sizeof(HGroup));
+        put(p->d_rdims, p->rd.data(), ndims * sizeof(HRowDim));
         if (!rc) rc = qmcgb::raise_smem_limit((const void *)halton_rows_kernel, p->rows_smem, "halton_rows_kernel smem");
     }
     put(p->d_req, p->hreq.data(), nreq * sizeof(HReq));
@@ -922,6 +926,7 @@ int qmc_halton_batch_create(const qmc_halton_request *reqs, int nreq, qmc_halton
     p->P.order = (const u16 *)p->d_order;
     p->P.wstart = (const u32 *)p->d_wstart;
     p->P.groups = (const HGroup *)p->d_groups;
+    p->P.rdims = (const HRowDim *)p->d_rdims;
     p->P.ngroups = (u32)groups.size();
     p->P.Cn = (const u32 *)p->d_Cn;
     p->P.mul = (const u32 *)p->d_mul;
@@ -1005,7 +1010,7 @@ int qmc_halton_plan_destroy(qmc_halton_plan *p)
     if (!p) return QMC_OK;
     drop_graph(p);
     for (void *q : {p->d_req, p->d_dims, p->d_C, p->d_Y, p->d_recip, p->d_tail, p->d_order, p->d_wstart, p->d_prep,
-                    p->d_groups, p->d_Cn, p->d_mul, p->d_flags, p->d_info})
+                    p->d_groups, p->d_rdims, p->d_Cn, p->d_mul, p->d_flags, p->d_info})
         if (q) cudaFree(q);
     delete p;
     return QMC_OK;

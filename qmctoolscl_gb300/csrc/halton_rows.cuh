@@ -64,6 +64,13 @@ struct HGroup {
     u32 h_size[HR_DIMS];  // per warp
 };
 
+// What this kernel needs of a dimension beyond HDim.
+struct HRowDim {
+    u32 t1, rows;  // FP64 rows at the front, rows that can change a sum of at least 2^-10
+    u32 K2, bK2;   // low digits of its index split, b^K2
+    u64 fdK2_M;
+};
+
 // what the preparation found about (l, j)
 __device__ __forceinline__ u32 hr_info(u32 t1, u32 tr, u32 rows, bool low_table)
 {
@@ -126,16 +133,17 @@ __global__ void halton_info_kernel(HPlanDev P, const u32 *flags, const u32 *Cn, 
         const HReq &R = P.req[req_of(P.req, P.nreq, w, [](const HReq &q) { return q.tl_base; })];
         const u64 loc = w - R.tl_base, l = loc / R.d, j = loc % R.d;
         const HDim &D = P.dims[R.dim0 + j];
+        const HRowDim &X = P.rdims[R.dim0 + j];
         const u32 *f = flags + R.t_base + l * R.s_per_l + D.s_off;
         const u32 *c0 = Cn + R.c_base + l * R.c_per_l + D.c_off;
-        bool wide = false, low = D.K2 > 1;
-        u32 tr = D.t1;
+        bool wide = false, low = X.K2 > 1;
+        u32 tr = X.t1;
         for (u32 t = 0; t < D.tmax; t++) {
             wide = wide || (f[t] & 2u);
-            if (t >= D.t1 && t < D.rows && (f[t] & 1u)) tr = t + 1;
+            if (t >= X.t1 && t < X.rows && (f[t] & 1u)) tr = t + 1;
             low = low || c0[t] != 1u;
         }
-        info[w] = wide ? hr_info(D.tmax, D.tmax, D.tmax, low) : hr_info(D.t1, tr, D.rows, low);
+        info[w] = wide ? hr_info(D.tmax, D.tmax, D.tmax, low) : hr_info(X.t1, tr, X.rows, low);
     }
 }
 
@@ -160,9 +168,11 @@ struct HConst {
     u32 T, H, L, h0;  // addresses of the tables; H, h0: this warp's and its first hi
 };
 
-// What the plain chain of a point needs of a dimension, in shared memory.
+// What the sections and the plain chain of a point need of a dimension, in shared memory (pointers
+// kept in registers over the points' loop spilled others: 6.96 ms).
 struct HSlow {
     const HDim *D;
+    const HRowDim *X;
     const u64 *Y;
     const u32 *mul;
 };
@@ -281,6 +291,7 @@ __global__ void __launch_bounds__(HR_THREADS, 1) halton_rows_kernel(HPlanDev P)
     const HReq &R = P.req[G.req];
     const u64 loc = item - G.item0, l = loc / G.splits, split = loc % G.splits;
     const HDim *dims = P.dims + R.dim0 + G.j0;
+    const HRowDim *rdims = P.rdims + R.dim0 + G.j0;
     const u32 *Cnl = P.Cn + R.c_base + l * R.c_per_l;
     const u64 *Yl = P.Y + R.y_base + l * R.y_per_l;
     const u32 *mul_l = P.mul + R.t_base + l * R.s_per_l;
@@ -306,7 +317,7 @@ __global__ void __launch_bounds__(HR_THREADS, 1) halton_rows_kernel(HPlanDev P)
                 T[t * b + g] = t >= t1 ? F | (exact ? 0u : 1u) : y;
             }
         }
-        if (tid == 0) slow[q] = HSlow{&D, Y, mul};
+        if (tid == 0) slow[q] = HSlow{&D, rdims + q, Y, mul};
         u32 *Cs = (u32 *)(sm + G.c_off[q]);
         for (u32 e = tid; e < D.mmax * tmax; e += nt) Cs[e] = Cnl[D.c_off + e];
     }
@@ -314,13 +325,14 @@ __global__ void __launch_bounds__(HR_THREADS, 1) halton_rows_kernel(HPlanDev P)
     for (u32 q = 0; q < nd; q++) {
         if (!(info_l[q] >> 31)) continue;
         const HDim &D = dims[q];
+        const HRowDim &X = rdims[q];
         const u32 pitch = D.tmax | 1u;
         const u32 *Cs = (const u32 *)(sm + G.c_off[q]);
         u16 *L = (u16 *)(sm + G.l_off[q]);
-        for (u32 x = warp; x < D.bK2; x += nw)
+        for (u32 x = warp; x < X.bK2; x += nw)
             for (u32 t = lane; t < D.tmax; t += 32) {
                 u32 acc = 0, h = x;
-                for (u32 k = 0; k < D.K2 && k < D.mmax; k++) {
+                for (u32 k = 0; k < X.K2 && k < D.mmax; k++) {
                     const u32 d = hdiv(D.fd_M, h);
                     acc += (h - d * D.b) * Cs[k * D.tmax + t];
                     h = d;
@@ -342,18 +354,19 @@ __global__ void __launch_bounds__(HR_THREADS, 1) halton_rows_kernel(HPlanDev P)
         __syncwarp();  // the sums of the section before have been read
         if (lane == 0) outs[warp] = R.x + (l * R.n + i0) * R.d + G.j0;
         for (u32 q = 0; q < nd; q++) {
-            const HDim &D = dims[q];
-            const u32 tmax = D.tmax, pitch = tmax | 1u, h0 = hdiv(D.fdK2_M, base);
-            const u32 nh = hdiv(D.fdK2_M, base + cnt - 1) - h0 + 1;
+            const HDim &D = *slow[q].D;
+            const HRowDim &X = *slow[q].X;
+            const u32 tmax = D.tmax, pitch = tmax | 1u, h0 = hdiv(X.fdK2_M, base);
+            const u32 nh = hdiv(X.fdK2_M, base + cnt - 1) - h0 + 1;
             const u32 *Cs = (const u32 *)(sm + G.c_off[q]);
             u16 *H = (u16 *)(sm + G.h_off[q] + warp * G.h_size[q]);
             if (lane == 0)
-                hc[q] = HConst{info_l[q], 8 * D.b, D.bK2, 2 * pitch, D.fdK2_M, sa + G.t_off[q],
+                hc[q] = HConst{info_l[q], 8 * D.b, X.bK2, 2 * pitch, X.fdK2_M, sa + G.t_off[q],
                                sa + G.h_off[q] + warp * G.h_size[q], sa + G.l_off[q], h0};
             for (u32 e = lane; e < nh * tmax; e += 32) {
                 const u32 u = e / tmax, t = e - u * tmax;
                 u32 acc = 0, h = h0 + u;
-                for (u32 k = D.K2; h && k < D.mmax; k++) {
+                for (u32 k = X.K2; h && k < D.mmax; k++) {
                     const u32 d = hdiv(D.fd_M, h);
                     acc += (h - d * D.b) * Cs[k * tmax + t];
                     h = d;
