@@ -1210,7 +1210,7 @@ def run_halton(args):
     cpu_pts = sum(p[2] for p in pieces)
     pts = r * n
     alg = 8.0 * r * n * d
-    fp64_r8 = profiled_value("halton_gen_kernel_r32_n2p18_d100.md", "fp64_warp_inst_per_launch_r8")
+    fp64_inst = profiled_value("halton_rows_kernel_r32_n2p18_d100.md", "fp64_warp_inst_per_launch")
     return {"metric": METRIC, "value": pts / (ms_fused / 1e3), "unit": "points/s", "n_gpus": 1,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_fused, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None, "dtype": "u32 digits, f64 adds (split FP64 unit / integer by the tuned share)",
@@ -1219,15 +1219,16 @@ def run_halton(args):
                                    "tmax_j=ceil(64/log2 b), LMS + permutation + digital shift + float "
                                    "(fused plan: prepare + generate)", "r": r, "n": n, "d": d,
                        "l2": "6.7 GB output per step >> 129 MB L2, no flush needed"},
-            "roofline": dict(roofline(alg, ms_gen), kernel="halton_gen_kernel",
-                             traffic=profiled_traffic("halton_gen_kernel_r32_n2p18_d100.md"),
-                             note="generation kernel alone; bound by the FP64 unit's digit adds (one per digit, "
-                                  "the FP64 pipe about 70 % busy in the ncu capture) and integer issue, not HBM"),
+            "roofline": dict(roofline(alg, ms_gen), kernel="halton_rows_kernel",
+                             traffic=profiled_traffic("halton_rows_kernel_r32_n2p18_d100.md"),
+                             note="generation kernel alone; bound by issue and the shared-memory pipe (73 and 79 % "
+                                  "in the ncu capture; the FP64 pipe 45 %: the digits after the first 16 bits are "
+                                  "added in integers), not HBM"),
             "fp64_roofline": dict(fp64_roofline(
-                None if fp64_r8 is None else fp64_r8 * r / 8.0, ms_gen, clk.get("sm_mhz")) or {},
+                None if fp64_inst is None else fp64_inst * r / 32.0, ms_gen, clk.get("sm_mhz")) or {},
                 note="generation kernel against the FP64 pipe's issue rate (2 lanes per SM per clock at the median "
-                     "SM clock sampled while timing); executed FP64 instructions from the ncu capture of the r=8 case "
-                     "in profiles/halton_gen_kernel_r32_n2p18_d100.md, scaled by r/8"),
+                     "SM clock sampled while timing); executed FP64 instructions from the ncu capture "
+                     "in profiles/halton_rows_kernel_r32_n2p18_d100.md"),
             "generate_only_ms": ms_gen,
             "uneven_batch": {"requests": 64, "points": upoints, "coords": ucoords, "graph_ms": ms_u_graph,
                              "per_request_plans_ms": ms_u_single, "speedup": ms_u_single / ms_u_graph,
@@ -1436,10 +1437,10 @@ def run_qrng(args):
             "config": {"workload": "halton_qrng, generalized, n=2^%d, d=100 (first 100 primes)" % (n.bit_length() - 1),
                        "n": n, "d": d, "l2": "%.0f MB output per step" % (8 * n * d / 1e6)},
             "roofline": dict(roofline(8.0 * n * d, ms), kernel="halton_qrng_kernel",
-                             note="bound by instruction issue on two units, not by HBM: each digit step is the "
-                                  "reference's rounded add and divide, a quarter of the warps on the FP64 pipe and "
-                                  "the rest in integer arithmetic (ncu: FP64 pipe 64 %, ALU 63 %, issue 76 %; "
-                                  "profiles/halton_qrng_kernel_n2p20_d100.md)"),
+                             note="bound by instruction issue on two units, not by HBM: about one step a point (the "
+                                  "values of the high digits are shared), the reference's rounded add and divide, half "
+                                  "of the steps on the FP64 pipe and half in integer arithmetic (ncu: FP64 pipe 71 %, "
+                                  "ALU 62 %; profiles/halton_qrng_kernel_n2p20_d100.md)"),
             "gpu_launches": args.steps,
             "cpu_baseline": {"value": ns / t_cpu, "unit": "points/s (d=100)", "cores": threads, "kind": "port",
                              "sample": "2^%d points of all 100 dimensions, one dimension per thread, by the oracle "
