@@ -10,7 +10,7 @@
 // m = gray(n_start+i)) is the XOR of the generating-matrix columns picked by
 // the set bits of m -- the closed form of the reference's recurrence.  A CTA
 // stages, for one randomisation and a tile of up to 64 columns, the table
-// T[lo][c] of XORs for the K low index bits (built by doubling) and the
+// T[lo][c] of XORs for the K low index bits (built in two steps) and the
 // columns H[b][c] for the high bits.  A coordinate is then T[m mod 2^K] ^
 // (XOR of H over the set bits of m >> K), the second term changing only every
 // 2^K rows.  The digital shift (x << ls) ^ s distributes over XOR and is
