@@ -15,7 +15,7 @@
 // (natural order: m = n_start+k; Gray order: m = gray(n_start+i)).  Each CTA
 // owns one randomisation, a column tile and a run of rows.  It stages in
 // shared memory a table T[lo][c] = XOR of the columns picked by the K low
-// bits lo, built by doubling from the generating matrix, plus the columns
+// bits lo, built in two steps from the generating matrix, plus the columns
 // for the high bits.  A point is then T[m mod 2^K] XOR H[m >> K], where H
 // (the XOR over the high bits) is recomputed only when m >> K changes -- one
 // shared-memory load and one XOR per coordinate, independent of the number

@@ -47,7 +47,7 @@
 // is staged in shared memory and stored as contiguous rows.  The grid holds
 // exactly the CTAs resident at once, striding over the equal-cost tiles.
 // Plans of a few million coordinates and more into device memory whose tables fit shared memory generate
-// with halton_rows_kernel (halton_rows.cuh) instead: first 100 primes, r=32, n=2^18, 20.3 -> 6.85 ms, bound by
+// with halton_rows_kernel (halton_rows.cuh) instead: first 100 primes, r=32, n=2^18, 20.3 -> 6.70 ms, bound by
 // issue and shared memory (73 and 79 %; FP64 45 %) where this kernel waits for the FP64 unit.
 #include <algorithm>
 #include <cmath>
@@ -664,7 +664,7 @@ void plan_rows(qmc_halton_plan *p, std::vector<HGroup> &groups)
             while (j < R.d && G.nd < HR_DIMS && (G.nd == 0 || j % HR_DIMS)) {
                 const HDim &h = p->hd[R.dim0 + j];
                 const HRowDim &rd = p->rd[R.dim0 + j];
-                const size_t pitch = 2 * (h.tmax | 1u), hs = up(((32 * HR_RUN - 1) / rd.bK2 + 2) * pitch);
+                const size_t pitch = 2 * hr_pitch(h.tmax), hs = up(((32 * HR_RUN - 1) / rd.bK2 + 2) * pitch);
                 const size_t T = up((size_t)h.tmax * h.b * 8), L = up(rd.bK2 * pitch), H = hs * (nt / 32),
                              C = up((size_t)h.mmax * h.tmax * 4);
                 if (used + T + L + H + C > HR_MAX_SMEM) break;

@@ -30,7 +30,7 @@
 // two thirds of the time).  The term tables serve all sections of the CTA, the sums H one.
 //
 // What bounds it: issue (73 % of the slots), the shared-memory pipe (79 %: a table read is two
-// wavefronts, a 32-byte piece of 32 rows up to 32) and the ALU (58 %).  First 100 primes, r = 32, n = 2^18: 6.85 ms
+// wavefronts, a 32-byte piece of 32 rows up to 32) and the ALU (58 %).  First 100 primes, r = 32, n = 2^18: 6.70 ms
 // (all FP64 adds 20.3; one section per CTA, and registers spilled for what the redone points need, 8.07).  The
 // stores alone, a CTA after another in a column of 32 bytes, take 4.4 ms; with the CTAs of a row next
 // to each other 2.6, but the whole no less (6.99: its CTAs differ in length).
@@ -41,7 +41,7 @@ namespace {
 constexpr u32 HR_DIMS = 4;
 constexpr u32 HR_PTS = 2;          // points of a lane: 32 apart
 constexpr u32 HR_THREADS = 1024;   // 64 registers: 8.0 ms; 768 threads 8.8, 4 points on 640 threads 9.0 (first 100
-                                   // primes, r=32, n=2^18; 4 dimensions unrolled 8.9: instruction cache)
+                                   // primes, r=32, n=2^18, one section; 4 dimensions unrolled 8.9: instruction cache)
 constexpr u32 HR_RUN = 16;         // most times 32 points in a warp's run (8: 7.21 ms, 16: 6.85, 32: 6.77, more memory)
 constexpr u32 HR_STEPS = 64;       // most times HR_THREADS points of a CTA (16: 7.86 ms, 64: 6.92, 128: 7.02)
 constexpr u32 HR_TINY = 9;         // integer rows need v >= 2^-(HR_TINY + 1)
@@ -50,7 +50,7 @@ constexpr u32 HR_HEAD_BITS = 16;   // b^t1 >= 2^16
 // Below these the warp kernel, which has no tables to set up, finishes sooner.  us of preparation and run,
 // warp kernel / this one, (r, n, d): (1, 20000, 20) 90 / 154, (4, 16384, 10) 121 / 157, (2, 30000, 50) 177 / 169,
 // (16, 8192, 20) 197 / 181, (1, 10^6, 3) 647 / 339; of the run: (300, 1024, 100) 768 / 1386, (256, 2048, 100)
-// 1267 / 1560, (32, 4096, 50) 211 / 185, (128, 4096, 100) 1266 / 979, (32, 262144, 100) 20320 / 6850, 64 uneven
+// 1267 / 1560, (32, 4096, 50) 211 / 185, (128, 4096, 100) 1266 / 979, (32, 262144, 100) 20320 / 6700, 64 uneven
 // requests of 73 M coordinates 3027 / 1489.
 constexpr double HR_MIN_COORDS = 2.4e6, HR_MIN_POINTS = 4000;
 constexpr u32 HR_MAX_SMEM = 216 * 1024;  // and 6 KB of HConst, HSlow and output rows
@@ -70,6 +70,9 @@ struct HRowDim {
     u32 K2, bK2;   // low digits of its index split, b^K2
     u64 fdK2_M;
 };
+
+// 16-bit entries of a row of H or L: an even count, two digits to a word, an odd number of words
+__host__ __device__ __forceinline__ u32 hr_pitch(u32 tmax) { return 2 * (((tmax + 1) / 2) | 1u); }
 
 // what the preparation found about (l, j)
 __device__ __forceinline__ u32 hr_info(u32 t1, u32 tr, u32 rows, bool low_table)
@@ -154,6 +157,12 @@ __device__ __forceinline__ u32 hr_ld16(u32 a)
     asm("{.reg .u16 h; ld.shared.u16 h, [%1]; cvt.u32.u16 %0, h;}" : "=r"(v) : "r"(a));
     return v;
 }
+__device__ __forceinline__ u32 hr_ld32(u32 a)
+{
+    u32 v;
+    asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+}
 __device__ __forceinline__ u64 hr_ld64(u32 a)
 {
     u64 v;
@@ -186,6 +195,13 @@ struct HDigits {
     {
         const u32 s = hr_ld16(hp + 2 * t) + (LOW ? hr_ld16(low + 2 * t) : low);
         return __viaddmin_u32(s, 0u - b8, s);
+    }
+    // rows t (even) and t + 1 in the halves of a word, both sums below 2^15: a read, an add and a
+    // conditional subtract for two digits (one each: 6.85 ms, 6.70 by pairs)
+    __device__ __forceinline__ u32 pair(u32 t, u32 b8) const
+    {
+        const u32 s = hr_ld32(hp + 2 * t) + (LOW ? hr_ld32(low + 2 * t) : low * 0x10001u);
+        return __viaddmin_u16x2(s, (0x10000u - b8) * 0x10001u, s);
     }
 };
 
@@ -236,12 +252,24 @@ __device__ __forceinline__ void hr_values(const HDigits<LOW> (&W)[HR_PTS], u32 T
 #pragma unroll
         for (u32 p = 0; p < HR_PTS; p++) acc[p] = dsum::add_even(acc[p], hr_ld64(T + W[p].at(t, b8)), half[p]);
     }
-#pragma unroll 2
-    for (; t < rows; t++) {
+    auto plain_row = [&]() {
         T += b8;
 #pragma unroll
         for (u32 p = 0; p < HR_PTS; p++) acc[p] = dsum::add_plain(acc[p], hr_ld64(T + W[p].at(t, b8)), half[p]);
+        t++;
+    };
+    if ((t & 1u) && t < rows) plain_row();
+#pragma unroll 1
+    for (; t + 1 < rows; t += 2) {
+        T += 2 * b8;
+#pragma unroll
+        for (u32 p = 0; p < HR_PTS; p++) {
+            const u32 m = W[p].pair(t, b8);
+            acc[p] = dsum::add_plain(acc[p], hr_ld64(T - b8 + (m & 0xFFFFu)), half[p]);
+            acc[p] = dsum::add_plain(acc[p], hr_ld64(T + (m >> 16)), half[p]);
+        }
     }
+    if (t < rows) plain_row();
 #pragma unroll
     for (u32 p = 0; p < HR_PTS; p++) {
         const u64 vb = as_bits(v[p]);
@@ -326,7 +354,7 @@ __global__ void __launch_bounds__(HR_THREADS, 1) halton_rows_kernel(HPlanDev P)
         if (!(info_l[q] >> 31)) continue;
         const HDim &D = dims[q];
         const HRowDim &X = rdims[q];
-        const u32 pitch = D.tmax | 1u;
+        const u32 pitch = hr_pitch(D.tmax);
         const u32 *Cs = (const u32 *)(sm + G.c_off[q]);
         u16 *L = (u16 *)(sm + G.l_off[q]);
         for (u32 x = warp; x < X.bK2; x += nw)
@@ -356,7 +384,7 @@ __global__ void __launch_bounds__(HR_THREADS, 1) halton_rows_kernel(HPlanDev P)
         for (u32 q = 0; q < nd; q++) {
             const HDim &D = *slow[q].D;
             const HRowDim &X = *slow[q].X;
-            const u32 tmax = D.tmax, pitch = tmax | 1u, h0 = hdiv(X.fdK2_M, base);
+            const u32 tmax = D.tmax, pitch = hr_pitch(tmax), h0 = hdiv(X.fdK2_M, base);
             const u32 nh = hdiv(X.fdK2_M, base + cnt - 1) - h0 + 1;
             const u32 *Cs = (const u32 *)(sm + G.c_off[q]);
             u16 *H = (u16 *)(sm + G.h_off[q] + warp * G.h_size[q]);
