@@ -47,7 +47,7 @@
 // is staged in shared memory and stored as contiguous rows.  The grid holds
 // exactly the CTAs resident at once, striding over the equal-cost tiles.
 // Plans of a few million coordinates and more into device memory whose tables fit shared memory generate
-// with halton_rows_kernel (halton_rows.cuh) instead: first 100 primes, r=32, n=2^18, 20.3 -> 6.70 ms, bound by
+// with halton_rows_kernel (halton_rows.cuh) instead: first 100 primes, r=32, n=2^18, 20.3 -> 6.67 ms, bound by
 // issue and shared memory (73 and 79 %; FP64 45 %) where this kernel waits for the FP64 unit.
 #include <algorithm>
 #include <cmath>

@@ -30,7 +30,7 @@
 // two thirds of the time).  The term tables serve all sections of the CTA, the sums H one.
 //
 // What bounds it: issue (73 % of the slots), the shared-memory pipe (79 %: a table read is two
-// wavefronts, a 32-byte piece of 32 rows up to 32) and the ALU (58 %).  First 100 primes, r = 32, n = 2^18: 6.70 ms
+// wavefronts, a 32-byte piece of 32 rows up to 32) and the ALU (58 %).  First 100 primes, r = 32, n = 2^18: 6.67 ms
 // (all FP64 adds 20.3; one section per CTA, and registers spilled for what the redone points need, 8.07).  The
 // stores alone, a CTA after another in a column of 32 bytes, take 4.4 ms; with the CTAs of a row next
 // to each other 2.6, but the whole no less (6.99: its CTAs differ in length).
@@ -50,7 +50,7 @@ constexpr u32 HR_HEAD_BITS = 16;   // b^t1 >= 2^16
 // Below these the warp kernel, which has no tables to set up, finishes sooner.  us of preparation and run,
 // warp kernel / this one, (r, n, d): (1, 20000, 20) 90 / 154, (4, 16384, 10) 121 / 157, (2, 30000, 50) 177 / 169,
 // (16, 8192, 20) 197 / 181, (1, 10^6, 3) 647 / 339; of the run: (300, 1024, 100) 768 / 1386, (256, 2048, 100)
-// 1267 / 1560, (32, 4096, 50) 211 / 185, (128, 4096, 100) 1266 / 979, (32, 262144, 100) 20320 / 6700, 64 uneven
+// 1267 / 1560, (32, 4096, 50) 211 / 185, (128, 4096, 100) 1266 / 979, (32, 262144, 100) 20320 / 6670, 64 uneven
 // requests of 73 M coordinates 3027 / 1489.
 constexpr double HR_MIN_COORDS = 2.4e6, HR_MIN_POINTS = 4000;
 constexpr u32 HR_MAX_SMEM = 216 * 1024;  // and 6 KB of HConst, HSlow and output rows
@@ -197,7 +197,7 @@ struct HDigits {
         return __viaddmin_u32(s, 0u - b8, s);
     }
     // rows t (even) and t + 1 in the halves of a word, both sums below 2^15: a read, an add and a
-    // conditional subtract for two digits (one each: 6.85 ms, 6.70 by pairs)
+    // conditional subtract for two digits (one each: 6.85 ms, 6.67 by pairs)
     __device__ __forceinline__ u32 pair(u32 t, u32 b8) const
     {
         const u32 s = hr_ld32(hp + 2 * t) + (LOW ? hr_ld32(low + 2 * t) : low * 0x10001u);
@@ -226,12 +226,18 @@ __device__ __forceinline__ void hr_values(const HDigits<LOW> (&W)[HR_PTS], u32 T
                                           double (&v)[HR_PTS], bool (&ok)[HR_PTS])
 {
     const u32 t1 = info & 1023u, tr = info >> 10 & 1023u, rows = info >> 20 & 1023u;
+    u32 t = t1 > 1 ? 2 : 1;  // one row where there are no more digits
 #pragma unroll
     for (u32 p = 0; p < HR_PTS; p++) {
-        v[p] = as_double(hr_ld64(T + W[p].at(0, b8)));
         ok[p] = true;
+        if (t == 2) {
+            const u32 m = W[p].pair(0, b8);
+            v[p] = __dadd_rn(as_double(hr_ld64(T + (m & 0xFFFFu))), as_double(hr_ld64(T + b8 + (m >> 16))));
+        } else {
+            v[p] = as_double(hr_ld64(T + W[p].at(0, b8)));
+        }
     }
-    u32 t = 1;
+    T += (t - 1) * b8;
     for (; t < t1; t++) {
         T += b8;
 #pragma unroll
