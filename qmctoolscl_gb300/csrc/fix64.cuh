@@ -32,7 +32,8 @@ typedef unsigned int u32;
 constexpr int TOP = 58;        // a group of stages starts below 2^TOP: 16 times that, times sqrt 2, fits
 constexpr int TOP_TW = 60;     // twiddle products that give a quarter start below 2^TOP_TW
 constexpr u32 E_MIN = 200;     // tiles whose largest biased exponent is outside
-constexpr u32 E_MAX = 1800;    // [E_MIN, E_MAX] (zeros, tiny, huge, inf, nan) stay in FP64
+constexpr u32 E_MAX = 1800;    // [E_MIN, E_MAX] (zeros, tiny, huge, inf, nan) stay in FP64,
+                               // before and after the scale: 60 bits below and 40 above stay normal
 
 FX_HD i64 make(u32 hi, u32 lo) { return (i64)(((u64)hi << 32) | lo); }
 FX_HD u32 hi32(i64 x) { return (u32)((u64)x >> 32); }

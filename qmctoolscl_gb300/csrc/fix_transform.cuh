@@ -263,13 +263,18 @@ __device__ __forceinline__ void halve_odd(T &x, bool odd)
     if (odd) x = fx::mul_real(x, fx::halves(fx::HALF));
 }
 
-__device__ __forceinline__ bool fix_range(u32 E) { return E >= fx::E_MIN && E <= fx::E_MAX; }
+// whether a tile of largest biased exponent E, written back times 2^scale_exp, keeps to fixed point
+__device__ __forceinline__ bool fix_range(u32 E, int scale_exp)
+{
+    const int s = (int)E + scale_exp;
+    return E >= fx::E_MIN && E <= fx::E_MAX && s >= (int)fx::E_MIN && s <= (int)fx::E_MAX;
+}
 
 // y * lam * f or y / lam * f (f = scale / n: the orthonormal factors of both transforms)
 __device__ __forceinline__ void pointwise(const PassArgs &a, u64 gi, double &yr, double &yi)
 {
     const u64 li = a.lam_all ? gi : (gi & ((1ull << a.m) - 1));
-    const double lr = a.lr[li], lm = a.li[li], f = a.lam_scale;
+    const double lr = a.lr[li], lm = a.li[li], f = a.fix_lam_scale;
     if (f != 1.0) {
         yr *= f;
         yi *= f;
@@ -287,7 +292,7 @@ __device__ __forceinline__ void pointwise(const PassArgs &a, u64 gi, double &yr,
 
 __device__ __forceinline__ double pointwise(const PassArgs &a, u64 gi, double y)
 {
-    const double l = a.lr[a.lam_all ? gi : (gi & ((1ull << a.m) - 1))], f = a.lam_scale;
+    const double l = a.lr[a.lam_all ? gi : (gi & ((1ull << a.m) - 1))], f = a.fix_lam_scale;
     if (f == 1.0) return a.divide ? y / l : y * l;
     return a.divide ? y * f / l : y * l * f;
 }
@@ -338,7 +343,7 @@ __global__ void __launch_bounds__(1 << (P - 4), P == 12 ? 2 : (P == 11 ? 4 : (P 
             prefetch_l2(a.xi + (next << P) + t * 16);
         }
         u32 E = get_max(ws[0]) >> 20;
-        if (!fix_range(E)) {
+        if (!fix_range(E, 0)) {
             fp64_tile<KIND>(a, sm, base, 0, 0, 1, TILE);
             continue;
         }
@@ -372,7 +377,7 @@ __global__ void __launch_bounds__(1 << (P - 4), P == 12 ? 2 : (P == 11 ? 4 : (P 
             put_max(ws[3], m2);
             __syncthreads();
             E = get_max(ws[3]) >> 20;
-            if (!fix_range(E)) {
+            if (!fix_range(E, a.scale_exp)) {
                 fp64_tile<KIND>(a, sm, base, 0, 0, 1, TILE);
                 continue;
             }
@@ -467,7 +472,7 @@ __global__ void __launch_bounds__(256, 2) fix_high_kernel(PassArgs a)
             prefetch_l2(a.xi + nb);
         }
         u32 E = mx >> 20;
-        bool bad = !fix_range(E);
+        bool bad = !fix_range(E, 0);
         if (S == 4) bad = __syncthreads_or(bad);
         if (bad) {
             fp64_tile<KIND>(a, sm, base, tile / chunks, c0, CT, 4096);
@@ -506,7 +511,7 @@ __global__ void __launch_bounds__(256, 2) fix_high_kernel(PassArgs a)
                 m2 = get_max(ws[2]);
             }
             E = m2 >> 20;
-            bad = !fix_range(E);
+            bad = !fix_range(E, a.scale_exp);
             if (S == 4) bad = __syncthreads_or(bad);
             if (bad) {
                 fp64_tile<KIND>(a, sm, base, tile / chunks, c0, CT, 4096);
@@ -577,7 +582,7 @@ __global__ void __launch_bounds__(1 << (P - 4), P == 12 ? 4 : (P == 11 ? 8 : (P 
         const u64 next = tile + gridDim.x;
         if (next < tiles) prefetch_l2(a.xr + (next << P) + t * 16);
         u32 E = get_max(ws[0]) >> 20;
-        if (!fix_range(E)) {
+        if (!fix_range(E, 0)) {
             fp64_tile<KIND>(a, sm, base, 0, 0, 1, TILE);
             continue;
         }
@@ -600,7 +605,7 @@ __global__ void __launch_bounds__(1 << (P - 4), P == 12 ? 4 : (P == 11 ? 8 : (P 
             put_max(ws[3], m2);
             __syncthreads();
             E = get_max(ws[3]) >> 20;
-            if (!fix_range(E)) {
+            if (!fix_range(E, a.scale_exp)) {
                 fp64_tile<KIND>(a, sm, base, 0, 0, 1, TILE);
                 continue;
             }
@@ -658,7 +663,7 @@ __global__ void __launch_bounds__(256, 4) fix_high_wht_kernel(PassArgs a)
             prefetch_l2(a.xr + ((next / chunks) << a.k1) + (next % chunks) * CT +
                         (S == 8 ? (u64)t << a.k0 : ((u64)(t >> 4) << a.k0) + (t & 15u) * 16u));
         u32 E = mx >> 20;
-        bool bad = !fix_range(E);
+        bool bad = !fix_range(E, 0);
         if (S == 4) bad = __syncthreads_or(bad);
         if (bad) {
             fp64_tile<KIND>(a, sm, base, tile / chunks, c0, CT, 4096);
@@ -686,7 +691,7 @@ __global__ void __launch_bounds__(256, 4) fix_high_wht_kernel(PassArgs a)
                 m2 = get_max(ws[2]);
             }
             E = m2 >> 20;
-            bad = !fix_range(E);
+            bad = !fix_range(E, a.scale_exp);
             if (S == 4) bad = __syncthreads_or(bad);
             if (bad) {
                 fp64_tile<KIND>(a, sm, base, tile / chunks, c0, CT, 4096);

@@ -96,9 +96,11 @@ struct PassArgs {
     const double *lr, *li;
     u32 lam_all, divide;
     double lam_scale;
-    // the fixed-point passes: the write-back scale as 2^scale_exp (times sqrt(1/2)); conj: the
-    // inverse steps read the forward transform's table
+    // the fixed-point passes: the write-back scale as 2^scale_exp (times sqrt(1/2)), and what of
+    // lam_scale that leaves to the pointwise step; conj: the inverse steps read the forward
+    // transform's table
     int scale_exp;
+    double fix_lam_scale;
     bool scale_odd, conj;
 };
 
@@ -601,13 +603,16 @@ int run_fused(int kind, u64 d1, u64 d2, u64 n_half, double *twr, double *twi, co
         a.lam_all = (u32)lam_all;
         a.divide = divide ? 1u : 0u;
         a.lam_scale = scale / (double)n;
-        if (li_ == np - 1 && fixed) {  // a factor that is a power of two goes into the exponent
+        a.fix_lam_scale = a.lam_scale;
+        if (li_ == np - 1 && fixed) {
+            // a factor that is a power of two goes into the exponent; tiles that it would take out of
+            // the range (fix_range), and products that overflow without it, are done in FP64 with
+            // the factor in the pointwise step
             int ex = 0;
             const double f = frexp(a.lam_scale, &ex);
             if (f == 0.5 && ex > -900 && ex < 900) {
-                a.lam_scale = 1.0;
+                a.fix_lam_scale = 1.0;
                 a.scale_exp = ex - 1;
-                a.scale = ldexp(1.0, ex - 1);
             }
         }
         const u32 elems = (1u << (p.k1 - p.k0)) * p.ct;
