@@ -192,7 +192,9 @@ __global__ void __launch_bounds__(128) nus_stream_kernel(NusDims m, u64 *__restr
     __shared__ u64 buf[2][STREAM_STEPS][33];
     const u32 warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g0 = blockIdx.x * 32, g = g0 + lane;
     const u32 need = g < m.S ? info[g].outputs : 0;
-    const u32 most = __reduce_max_sync(0xFFFFFFFFu, need), least = __reduce_min_sync(0xFFFFFFFFu, need);
+    const u32 most = __reduce_max_sync(0xFFFFFFFFu, need);
+    // lanes past the last generator step a stream of zeros along with the others, into a column that no one reads
+    const u32 least = __reduce_min_sync(0xFFFFFFFFu, g < m.S ? need : NONE);
     u64 *st = states + (g < m.S ? m.s0 + g : 0) * 6;
     Sfc64 r{0, 0, 0, 0, 0, 0};
     if (warp == 0 && g < m.S) r = Sfc64{st[0], st[1], st[2], st[3], 0, 0};

@@ -54,3 +54,33 @@ def test_counters_near_their_upper_half(n):
     forest.close()
     assert np.array_equal(got, want)
     assert np.array_equal(_states(gens).reshape(-1), words)
+
+
+@pytest.mark.parametrize("d", [1, 10, 31, 32, 33, 37, 64, 70])
+@pytest.mark.parametrize("n", [300, 700])
+def test_generator_counts(d, n):
+    """Generators that fill the streams' warps and that leave lanes without one, over several blocks of
+    outputs, with counters that carry into their upper half at different blocks in different lanes, in one lane
+    only, and in none."""
+    import oracle
+    import qmctoolscl_gb300 as q
+    from .test_gpu_nus import _states
+    rng = np.random.Generator(np.random.SFC64(n + d))
+    gens = [np.random.Generator(np.random.SFC64(k)) for k in range(d)]
+    for k, g in enumerate(gens):
+        if k % 32 in (0, 5, 30) and k < 64:
+            state = g.bit_generator.state
+            state["state"]["state"][3] = np.uint64((1 << 32) * (k + 1) - (1 + 67 * (k % 32) // 5))
+            g.bit_generator.state = state
+    words = _states(gens).reshape(-1).copy()
+    xb = rng.integers(0, 1 << 63, (1, n, d), dtype=np.uint64) * np.uint64(2)
+    forest = oracle.NusForest(d)
+    roots = np.array([q.NUSNode_dnb2() for _ in range(d)]).reshape(1, d)
+    for part in (xb, xb[:, ::-1] ^ np.uint64(1 << 40)):
+        want, got = np.zeros((1, n, d), np.uint64), np.zeros((1, n, d), np.uint64)
+        part = np.ascontiguousarray(part)
+        forest.scramble(1, n, d, 1, 64, 64, words, part, want)
+        q.dnb2_nested_uniform_scramble(1, n, d, 1, 64, 64, np.array(gens, dtype=object).reshape(1, d), roots, part, got)
+        assert np.array_equal(got, want)
+        assert np.array_equal(_states(gens).reshape(-1), words)
+    forest.close()
