@@ -107,16 +107,7 @@ __global__ void __launch_bounds__(256) dnb2_run_kernel(u64 r, u64 words, u32 d, 
         auto one = [&](u64 w, u64 s) {
             return SHIFT ? (w << ls) ^ s : (u64)__double_as_longlong(to_float_bits(w, e));
         };
-        const u32 head = (u32)(((uintptr_t)dst >> 3) & 1u);
-        if ((((uintptr_t)src >> 3) & 1u) != head) {  // never both on a 16-byte boundary: word by word
-            u32 col = SHIFT ? (u32)(((u64)blockIdx.x * 256 + threadIdx.x) % d) : 0u;
-            const u32 cs = SHIFT ? (u32)(step % d) : 0u;
-            for (u64 w = (u64)blockIdx.x * 256 + threadIdx.x; w < words; w += step) {
-                __stcs(dst + w, one(__ldcs(src + w), SHIFT ? sh[col] : 0));
-                if (SHIFT) col = col + cs >= d ? col + cs - d : col + cs;
-            }
-            continue;
-        }
+        const u32 head = (u32)(((uintptr_t)dst >> 3) & 1u);  // src is on or off a 16-byte boundary like dst
         const u64 pairs = (words - head) / 2;
         const ulonglong2 *s2 = (const ulonglong2 *)(src + head);
         ulonglong2 *d2 = (ulonglong2 *)(dst + head);
@@ -312,10 +303,21 @@ Shape rows_shape(u64 r, u64 n, u64 ngroups)
 // Rows of pairs (vec2) that fill their block's threads keep the row kernels, which read each column's
 // shift once; others go as runs.  us, rows / runs, (r, n, d): shift (8, 100003, 21) 56.7 / 44.0,
 // (1, 20000, 127) 14.2 / 7.0, (8, 100003, 32) 62.4 / 65.8, (1, 1000, 5) 2.1 / 2.7; float 65.6 / 43.6,
-// 12.7 / 7.0, 63.5 / 64.9, 1.9 / 2.1.
-bool as_run(u64 words, u64 d, bool vec2)
+// 12.7 / 7.0, 63.5 / 64.9, 1.9 / 2.1.  A randomisation's run takes blocks of its own: short ones leave
+// their threads idle, and pay a staging each, unless all blocks fit the GPU at once, or rows are long.  Shift,
+// rows / runs: (16384, 16, 3) 24.9 / 37.2, (8192, 100, 6) 21.4 / 24.3, (2050, 341, 6) 9.2 / 9.3, (1024, 128, 5)
+// 5.7 / 4.9, (4112, 204, 5) 15.0 / 13.3, (11096, 6, 63) 30.3 / 29.5, (22192, 6, 126) 89.0 / 76.2; float 25.7 / 31.9,
+// 25.1 / 22.5, 13.7 / 10.1, 5.7 / 4.2, 17.8 / 13.0, 30.7 / 25.3, 88.2 / 70.6.
+// `together`: in and out of every randomisation are alike on or off a 16-byte boundary; otherwise there are no
+// pairs (8, 100003, 21: 59.4 / 73.8).
+bool as_run(u64 r, u64 n, u64 d, bool vec2, bool together, bool shift)
 {
-    if (words < (1ull << 17)) return false;  // a launch's latency either way, and no table to stage
+    if (r * n * d < (1ull << 17)) return false;  // a launch's latency either way, and no table to stage
+    if (!together) return false;
+    const bool one_wave = r <= (u64)qmcgb::sm_count() * 8;
+    const u64 least = shift ? (one_wave ? (vec2 ? 500 : 250) : d < 32 ? (vec2 ? 2000 : 1000) : vec2 ? 750 : 400)
+                            : (d >= 32 ? 0 : one_wave || vec2 ? 250 : 400);
+    if (n * d < least) return false;
     if (!vec2) return true;
     const u64 groups = d / 2;
     return groups < 32 ? (groups & (groups - 1)) != 0 : groups % 32 != 0;
@@ -465,7 +467,8 @@ int qmc_dnb2_digital_shift(uint64_t r, uint64_t n, uint64_t d, uint64_t r_x, con
     if (r == 0 || n == 0 || d == 0) return QMC_OK;
     QMC_REQUIRE(r_x > 0 && lshifts && xb && shiftsb && xrb, "bad r_x or null array pointer");
     const bool vec2 = d % 2 == 0 && aligned16(xb) && aligned16(xrb);
-    if (d < RUN_MAX_D && as_run(r * n * d, d, vec2)) {
+    const bool together = ((((uintptr_t)xb ^ (uintptr_t)xrb) >> 3) & 1u) == 0 && (r_x == r || (n * d) % 2 == 0);
+    if (d < RUN_MAX_D && as_run(r, n, d, vec2, together, true)) {
         dnb2_run_kernel<true><<<run_grid(r, n * d), 256, (d + 1) * sizeof(u64), QMC_STREAM(s)>>>(
             r, n * d, (u32)d, r_x, (const u64 *)lshifts, (const u64 *)xb, (const u64 *)shiftsb, (u64 *)xrb);
         return qmcgb::launch_status("dnb2_digital_shift");
@@ -488,7 +491,8 @@ int qmc_dnb2_integer_to_float(uint64_t r, uint64_t n, uint64_t d, const uint64_t
     if (r == 0 || n == 0 || d == 0) return QMC_OK;
     QMC_REQUIRE(tmaxes && xb && x, "null array pointer");
     const bool vec2 = d % 2 == 0 && aligned16(xb) && aligned16(x);
-    if (as_run(r * n * d, d, vec2)) {
+    const bool together = ((((uintptr_t)xb ^ (uintptr_t)x) >> 3) & 1u) == 0;
+    if (as_run(r, n, d, vec2, together, false)) {
         dnb2_run_kernel<false><<<run_grid(r, n * d), 256, 0, QMC_STREAM(s)>>>(
             r, n * d, 1u, 1, (const u64 *)tmaxes, (const u64 *)xb, nullptr, (u64 *)x);
         return qmcgb::launch_status("dnb2_integer_to_float");

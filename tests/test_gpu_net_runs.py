@@ -44,6 +44,15 @@ def test_runs(r, r_x, n, d, off_in, off_out):
     assert np.array_equal(_bits(gx), x.reshape(-1).view(U))
 
 
+@pytest.mark.parametrize("r,r_x,n,d", [(1300, 1300, 199, 5), (1300, 1, 201, 5), (1300, 1300, 333, 6), (1300, 650, 334, 6),
+                                       (1000, 1000, 49, 5), (1000, 1, 51, 5), (1000, 500, 83, 6), (1000, 2, 85, 6),
+                                       (70000, 35000, 1, 3), (70000, 70000, 2, 2)])
+@pytest.mark.parametrize("off_in,off_out", [(0, 0), (0, 1), (1, 1)])
+def test_many_randomisations(r, r_x, n, d, off_in, off_out):
+    """On both sides of the limits on a randomisation's words, and more randomisations than a grid has rows."""
+    test_runs(r, r_x, n, d, off_in, off_out)
+
+
 @pytest.mark.parametrize("mmax", [1, 2, 3, 5, 7, 8, 9, 17, 33, 64])
 @pytest.mark.parametrize("d", [1, 3, 8, 63, 64, 65])
 def test_tables(mmax, d):
