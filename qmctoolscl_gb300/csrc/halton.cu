@@ -558,13 +558,6 @@ void drop_graph(qmc_halton_plan *p)
 // of the warp kernel
 bool use_rows(const qmc_halton_plan *p) { return p->items && !p->mixed; }
 
-int tail_launch(qmc_halton_plan *p, cudaStream_t st)
-{
-    const unsigned cap = (unsigned)qmcgb::sm_count() * 16;
-    halton_tail_kernel<<<qmcgb::grid_for(p->P.titems, 128, cap), 128, 0, st>>>(p->P, (u32 *)p->d_tail);
-    return qmcgb::launch_status("halton_tail_kernel");
-}
-
 int prepare_launch(qmc_halton_plan *p, cudaStream_t st)
 {
     const unsigned cap = (unsigned)qmcgb::sm_count() * 16;
@@ -590,7 +583,10 @@ int prepare_launch(qmc_halton_plan *p, cudaStream_t st)
             p->P, (const u32 *)p->d_flags, (const u32 *)p->d_Cn, (u32 *)p->d_info);
         if (int rc = qmcgb::launch_status("halton_info_kernel")) return rc;
     }
-    return use_rows(p) ? QMC_OK : tail_launch(p, st);
+    // last, the warp kernel's stop table: also in plans that generate from the tables now, so that a
+    // preparation (or a graph of one) serves both kernels whatever share is set later
+    halton_tail_kernel<<<qmcgb::grid_for(p->P.titems, 128, cap), 128, 0, st>>>(p->P, (u32 *)p->d_tail);
+    return qmcgb::launch_status("halton_tail_kernel");
 }
 
 // Every tile costs the same, and the CTAs stride over the tiles: a grid of exactly the CTAs
@@ -995,14 +991,8 @@ int qmc_halton_plan_set_fp64_share(qmc_halton_plan *p, double share)
     if (int rc = qmcgb::cuda_status(cudaDeviceSynchronize(), "synchronise before rewriting the descriptors"))
         return rc;
     drop_graph(p);
-    if (int rc = qmcgb::cuda_status(
-            cudaMemcpy(p->d_dims, p->hd.data(), p->hd.size() * sizeof(HDim), cudaMemcpyHostToDevice), "copy"))
-        return rc;
-    if (!p->prepared || use_rows(p)) return QMC_OK;
-    // the warp kernel's stop table (a preparation for the other kernel left it out; a maximum over
-    // suffixes is its own maximum, so a second pass changes nothing)
-    if (int rc = tail_launch(p, nullptr)) return rc;
-    return qmcgb::cuda_status(cudaDeviceSynchronize(), "halton_tail_kernel");
+    return qmcgb::cuda_status(cudaMemcpy(p->d_dims, p->hd.data(), p->hd.size() * sizeof(HDim), cudaMemcpyHostToDevice),
+                              "copy");
 }
 
 int qmc_halton_plan_destroy(qmc_halton_plan *p)
