@@ -330,10 +330,17 @@ int qmc_plan_destroy(qmc_plan *plan);
  * below 2^32 (larger ones set bit 8 of the device error word).  Create
  * allocates the packed tables; prepare fills them from the arrays the dims
  * point to (read at that time, on the stream); run generates x.
- * set_fp64_share picks the share of the digit adds that run on the FP64
- * unit (the rest run in integer arithmetic, same bits either way), a tuning
- * knob for the balance between the two pipes (default 1.0: all FP64, the fastest
- * measured on GB300). */
+ * run has two kernels, same bits either way.  Plans of about 2.4 million
+ * coordinates and more into device memory whose tables fit shared memory
+ * generate from those tables (digits after the first 16 bits added in integers);
+ * others, and all outputs in pinned host memory, by warps that share an
+ * index's digits.  set_fp64_share is a tuning knob of the second kernel: the
+ * share of the digit adds that run on the FP64 unit, the rest in integer
+ * arithmetic.  1.0, the default, is the fastest measured there; a share below 1
+ * moves a plan of the first kernel to the second, about three times slower (first
+ * 100 primes, r = 32, n = 2^18: 6.7 and 20.3 ms).  info tells whether a plan has the
+ * tables, and whether run uses them at the present share (either pointer may be
+ * NULL). */
 typedef struct qmc_gdn_dim {
     uint64_t b, tmax, mmax;
     const uint64_t *S;      /* r * tmax * tmax scrambling matrices */
@@ -360,6 +367,7 @@ int qmc_halton_plan_run(qmc_halton_plan *plan, qmc_stream_t s);
  * legacy default stream); later calls replay it */
 int qmc_halton_plan_graph_launch(qmc_halton_plan *plan, qmc_stream_t s);
 int qmc_halton_plan_set_fp64_share(qmc_halton_plan *plan, double share);
+int qmc_halton_plan_info(const qmc_halton_plan *plan, int *has_tables, int *uses_tables);
 int qmc_halton_plan_destroy(qmc_halton_plan *plan);
 
 /* ---- one digital-net request without any allocation -------------------------

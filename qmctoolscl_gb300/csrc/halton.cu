@@ -995,6 +995,14 @@ int qmc_halton_plan_set_fp64_share(qmc_halton_plan *p, double share)
                               "copy");
 }
 
+int qmc_halton_plan_info(const qmc_halton_plan *p, int *has_tables, int *uses_tables)
+{
+    QMC_REQUIRE(p, "null plan");
+    if (has_tables) *has_tables = p->items != 0;
+    if (uses_tables) *uses_tables = use_rows(p);
+    return QMC_OK;
+}
+
 int qmc_halton_plan_destroy(qmc_halton_plan *p)
 {
     if (!p) return QMC_OK;

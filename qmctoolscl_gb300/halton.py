@@ -54,9 +54,10 @@ def _lib():
         L.qmc_halton_plan_graph_launch.argtypes = [_P, _P]
         L.qmc_halton_plan_destroy.argtypes = [_P]
         L.qmc_halton_plan_set_fp64_share.argtypes = [_P, _ct.c_double]
+        L.qmc_halton_plan_info.argtypes = [_P, _ct.POINTER(_ct.c_int), _ct.POINTER(_ct.c_int)]
         for fn in ("qmc_halton_plan_create", "qmc_halton_batch_create", "qmc_halton_plan_prepare",
                    "qmc_halton_plan_run", "qmc_halton_plan_graph_launch", "qmc_halton_plan_destroy",
-                   "qmc_halton_plan_set_fp64_share"):
+                   "qmc_halton_plan_set_fp64_share", "qmc_halton_plan_info"):
             getattr(L, fn).restype = _ct.c_int
         L._halton_bound = True
     return L
@@ -163,9 +164,18 @@ class HaltonBatch:
     def graph_launch(self, stream):
         _ffi.check(_lib().qmc_halton_plan_graph_launch(self._h, stream.cuda_stream), "halton_plan_graph_launch")
 
+    def info(self):
+        """dict(has_tables, uses_tables): whether the plan can generate from tables in shared memory (device
+        outputs, enough points, tables that fit), and whether run() does at the present share."""
+        has, uses = _ct.c_int(), _ct.c_int()
+        _ffi.check(_lib().qmc_halton_plan_info(self._h, _ct.byref(has), _ct.byref(uses)), "halton_plan_info")
+        return {"has_tables": bool(has.value), "uses_tables": bool(uses.value)}
+
     def set_fp64_share(self, share):
-        """Share of the digit adds run on the FP64 unit (the rest in integer
-        arithmetic); the results are the same bits either way."""
+        """For plans without tables (info()): the share of the digit adds run on the FP64
+        unit (the rest in integer arithmetic).  A share below 1 moves a plan that
+        has tables to that kernel, about three times slower.  The results are the
+        same bits either way."""
         _ffi.check(_lib().qmc_halton_plan_set_fp64_share(self._h, float(share)), "halton_plan_set_fp64_share")
         self.share = float(share)
 
