@@ -150,7 +150,9 @@ __global__ void halton_info_kernel(HPlanDev P, const u32 *flags, const u32 *Cn, 
     }
 }
 
-// Table reads by 32-bit shared-memory address (tables that no one writes after the last barrier).
+// Table reads by 32-bit shared-memory address.  hr_ld16, hr_ld32: T and L, which no one writes after the last
+// barrier.  The sums H are written anew in every section: their reads (hr_sum16, hr_sum32) stay
+// between the warp's barriers around the writes.
 __device__ __forceinline__ u32 hr_ld16(u32 a)
 {
     u32 v;
@@ -167,6 +169,18 @@ __device__ __forceinline__ u64 hr_ld64(u32 a)
 {
     u64 v;
     asm("ld.shared.u64 %0, [%1];" : "=l"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ u32 hr_sum16(u32 a)
+{
+    u32 v;
+    asm volatile("{.reg .u16 h; ld.shared.u16 h, [%1]; cvt.u32.u16 %0, h;}" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ u32 hr_sum32(u32 a)
+{
+    u32 v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
     return v;
 }
 
@@ -193,14 +207,14 @@ struct HDigits {
     u32 hp, low;  // H[hi]; L[x] or the low part itself, times 8
     __device__ __forceinline__ u32 at(u32 t, u32 b8) const
     {
-        const u32 s = hr_ld16(hp + 2 * t) + (LOW ? hr_ld16(low + 2 * t) : low);
+        const u32 s = hr_sum16(hp + 2 * t) + (LOW ? hr_ld16(low + 2 * t) : low);
         return __viaddmin_u32(s, 0u - b8, s);
     }
     // rows t (even) and t + 1 in the halves of a word, both sums below 2^15: a read, an add and a
     // conditional subtract for two digits (one each: 6.85 ms, 6.67 by pairs)
     __device__ __forceinline__ u32 pair(u32 t, u32 b8) const
     {
-        const u32 s = hr_ld32(hp + 2 * t) + (LOW ? hr_ld32(low + 2 * t) : low * 0x10001u);
+        const u32 s = hr_sum32(hp + 2 * t) + (LOW ? hr_ld32(low + 2 * t) : low * 0x10001u);
         return __viaddmin_u16x2(s, (0x10000u - b8) * 0x10001u, s);
     }
 };
