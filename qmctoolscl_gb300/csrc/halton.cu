@@ -895,8 +895,8 @@ int qmc_halton_batch_create(const qmc_halton_request *reqs, int nreq, qmc_halton
     alloc(&p->d_order, order.size() * sizeof(u16));
     alloc(&p->d_wstart, wstart.size() * sizeof(u32));
     alloc(&p->d_prep, ndims * sizeof(PrepDim));
-    alloc(&p->d_flags, t_base * sizeof(u32));
     if (p->items) {
+        alloc(&p->d_flags, t_base * sizeof(u32));
         alloc(&p->d_groups, groups.size() * sizeof(HGroup));
         alloc(&p->d_rdims, ndims * sizeof(HRowDim));
         alloc(&p->d_Cn, c_base * sizeof(u32));
