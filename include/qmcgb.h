@@ -311,6 +311,8 @@ int qmc_plan_graph_launch(qmc_plan *plan, qmc_stream_t s);
  * grab, coordinates per tile (rounded to whole rows); 0 keeps a value.  Drops any
  * captured graph. */
 int qmc_plan_set_tuning(qmc_plan *plan, int ctas_per_sm, int chunk, uint64_t tile_coords);
+/* the values in use (any pointer may be NULL); those of a new plan come from its size */
+int qmc_plan_get_tuning(const qmc_plan *plan, int *ctas_per_sm, int *chunk, uint64_t *tile_coords);
 /* tiles, coordinates and output bytes of one run, kernel launches per run */
 int qmc_plan_info(const qmc_plan *plan, uint64_t *tiles, uint64_t *coords, uint64_t *bytes_out, int *launches);
 int qmc_plan_destroy(qmc_plan *plan);

@@ -187,11 +187,12 @@ def _plan_lib():
         L.qmc_net_plan_create.argtypes = [_ct.POINTER(NetRequest), _ct.c_int, _ct.POINTER(_P)]
         L.qmc_lat_plan_create.argtypes = [_ct.POINTER(LatRequest), _ct.c_int, _ct.POINTER(_P)]
         for fn in ("qmc_net_plan_create", "qmc_lat_plan_create", "qmc_plan_run", "qmc_plan_graph_launch",
-                   "qmc_plan_set_tuning", "qmc_plan_info", "qmc_plan_destroy"):
+                   "qmc_plan_set_tuning", "qmc_plan_get_tuning", "qmc_plan_info", "qmc_plan_destroy"):
             getattr(L, fn).restype = _ct.c_int
         L.qmc_plan_run.argtypes = [_P, _P]
         L.qmc_plan_graph_launch.argtypes = [_P, _P]
         L.qmc_plan_set_tuning.argtypes = [_P, _ct.c_int, _ct.c_int, _U64]
+        L.qmc_plan_get_tuning.argtypes = [_P, _ct.POINTER(_ct.c_int), _ct.POINTER(_ct.c_int), _ct.POINTER(_U64)]
         L.qmc_plan_info.argtypes = [_P, _ct.POINTER(_U64), _ct.POINTER(_U64), _ct.POINTER(_U64),
                                     _ct.POINTER(_ct.c_int)]
         L.qmc_plan_destroy.argtypes = [_P]
@@ -256,6 +257,13 @@ class Plan:
         _ffi.check(_plan_lib().qmc_plan_set_tuning(self._h, int(ctas_per_sm), int(chunk), int(tile_coords)),
                    "plan_set_tuning")
         self.tuning = (ctas_per_sm, chunk, tile_coords)
+
+    def get_tuning(self):
+        """(ctas_per_sm, chunk, tile_coords) in use; a new plan's come from its size."""
+        ctas, chunk, tile = _ct.c_int(), _ct.c_int(), _U64()
+        _ffi.check(_plan_lib().qmc_plan_get_tuning(self._h, _ct.byref(ctas), _ct.byref(chunk), _ct.byref(tile)),
+                   "plan_get_tuning")
+        return ctas.value, chunk.value, tile.value
 
     def info(self):
         t, c, b, l_ = _U64(), _U64(), _U64(), _ct.c_int()
@@ -353,6 +361,9 @@ class LatPlan(Plan):
 # --------------------------------------------------------------------------
 # autotuner: launch shapes of the persistent kernel, cached per shape class
 
+# The cache's keys carry a number that goes up when the kernels change what a value means or
+# is worth: choices timed on other kernels are not applied.
+TUNE_VERSION = 2
 TUNE_CTAS = (2, 4, 8)
 TUNE_CHUNK = (1, 4, 16)
 TUNE_TILE = (1 << 14, 1 << 16, 1 << 18)
@@ -407,25 +418,24 @@ def time_plan(plan, stream, reps):
 
 
 def autotune(plan, stream=None, reps=3, use_cache=True):
-    """Try every (CTAs per SM, tiles per grab, coordinates per tile) of the
-    candidate grid on this plan, keep the fastest, and remember it for plans
-    of the same shape class.  Returns (ctas_per_sm, chunk, tile_coords, ms)."""
+    """Try the plan's present (CTAs per SM, tiles per grab, coordinates per tile)
+    and every one of the candidate grid on this plan, keep the fastest, and
+    remember it for plans of the same shape class.  Returns (ctas_per_sm, chunk, tile_coords, ms)."""
     torch = _t()
     stream = stream if stream is not None else torch.cuda.current_stream()
-    key = plan.shape_class()
+    key = "v%d|%s" % (TUNE_VERSION, plan.shape_class())
     if use_cache:
         hit = _load_cache().get(key)
         if hit:
             plan.set_tuning(*hit[:3])
             return tuple(hit)
     best = None
-    for tile in TUNE_TILE:
-        for ctas in TUNE_CTAS:
-            for chunk in TUNE_CHUNK:
-                plan.set_tuning(ctas, chunk, tile)
-                ms = time_plan(plan, stream, reps)
-                if best is None or ms < best[3]:
-                    best = (ctas, chunk, tile, ms)
+    grid = [(ctas, chunk, tile) for tile in TUNE_TILE for ctas in TUNE_CTAS for chunk in TUNE_CHUNK]
+    for shape in [tuple(plan.get_tuning())] + grid:
+        plan.set_tuning(*shape)
+        ms = time_plan(plan, stream, reps)
+        if best is None or ms < best[3]:
+            best = shape + (ms,)
     plan.set_tuning(*best[:3])
     if use_cache:
         _store_cache(key, list(best))

@@ -591,6 +591,15 @@ int qmc_plan_set_tuning(qmc_plan *p, int ctas_per_sm, int chunk, uint64_t tile_c
     return QMC_OK;
 }
 
+int qmc_plan_get_tuning(const qmc_plan *p, int *ctas_per_sm, int *chunk, uint64_t *tile_coords)
+{
+    QMC_REQUIRE(p, "null plan");
+    if (ctas_per_sm) *ctas_per_sm = p->ctas_per_sm;
+    if (chunk) *chunk = (int)p->chunk;
+    if (tile_coords) *tile_coords = p->tile_coords;
+    return QMC_OK;
+}
+
 int qmc_plan_info(const qmc_plan *p, uint64_t *tiles, uint64_t *coords, uint64_t *bytes_out, int *launches)
 {
     QMC_REQUIRE(p, "null plan");

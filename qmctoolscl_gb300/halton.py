@@ -181,12 +181,14 @@ class HaltonBatch:
 
     def tune(self, stream=None, shares=(0.0, 0.5, 0.75, 1.0), reps=3, use_cache=True):
         """Time run() at each FP64 share, keep the fastest, remember it for plans of the same
-        shape class (the autotuner cache of qmctoolscl_gb300.batch).  Returns (share, ms)."""
+        shape class and generation kernel (the autotuner cache of qmctoolscl_gb300.batch).  Returns
+        (share, ms)."""
         from . import batch
         torch = _torch()
         stream = stream if stream is not None else torch.cuda.current_stream()
-        key = "halton|coords2^%d|req2^%d|%s" % (int(np.log2(max(self.coords, 1))), int(np.log2(max(self.nreq, 1))),
-                                               batch._device_name())
+        key = "v%d|halton|tables%d|coords2^%d|req2^%d|%s" % (
+            batch.TUNE_VERSION, self.info()["has_tables"], int(np.log2(max(self.coords, 1))),
+            int(np.log2(max(self.nreq, 1))), batch._device_name())
         if use_cache:
             hit = batch._load_cache().get(key)
             if hit:
