@@ -1,12 +1,15 @@
 // fix64.cuh -- block fixed-point arithmetic of the FP64 transforms.
 //
 // GB300's FP64 unit takes two operations per SM and clock, its integer pipes
-// about 64, so the transforms hold a tile's values as 64-bit integers with one
-// common exponent: value = x * 2^e.  A tile enters with |x| < 2^58, five bits more
-// than a double's 53 for its largest values, and is shifted back under 2^58 before
-// every group of four stages (each at most doubles a value), so that no sum
-// overflows.  Adds are exact; a twiddle product (factors in units of 2^-62) is off by
-// about half a unit, 2^-59 of the tile's largest value.
+// about 64, so the transforms hold their values as 64-bit integers, value = x * 2^e.  The 16
+// values that a thread takes through a group of four stages share an exponent, at most 2^58 in
+// modulus on the way in: five bits more than a double's 53 for the largest of them.  Each stage at most
+// doubles a value, so that no sum overflows.  Adds are exact; a twiddle product (factors in units of
+// 2^-62) is off by about half a unit.  Between groups every thread collects 16 values of other
+// threads, and where they are far smaller than the tile's they take an exponent of their own
+// (common_exponent): what the stages before cancelled keeps the bits that it has, as in floating point.
+// One exponent per tile lost them beside the tile's largest sums (constant data plus 1e-12 of noise: the
+// outputs but the first had 5 digits).
 //
 // Everything here compiles for the host too (the CPU test holds it to 128-bit
 // integer arithmetic).
@@ -18,9 +21,11 @@
 #ifdef __CUDACC__
 #define FX_HD __host__ __device__ __forceinline__
 #define FX_UNROLL _Pragma("unroll")
+#define FX_UNROLL2 _Pragma("unroll 2")
 #else
 #define FX_HD inline
 #define FX_UNROLL
+#define FX_UNROLL2
 #endif
 
 namespace fx {
@@ -31,9 +36,11 @@ typedef unsigned int u32;
 
 constexpr int TOP = 58;        // a group of stages starts below 2^TOP: 16 times that, times sqrt 2, fits
 constexpr int TOP_TW = 60;     // twiddle products that give a quarter start below 2^TOP_TW
-constexpr u32 E_MIN = 200;     // tiles whose largest biased exponent is outside
-constexpr u32 E_MAX = 1800;    // [E_MIN, E_MAX] (zeros, tiny, huge, inf, nan) stay in FP64,
-                               // before and after the scale: 60 bits below and 40 above stay normal
+// Blocks of 16 whose largest biased exponent is outside [E_MIN, E_MAX] (tiny, huge, inf, nan),
+// before or after the scale, send their tile to FP64.
+constexpr u32 E_MIN = 200;
+constexpr u32 E_MAX = 1800;
+constexpr int E_ZERO = -4000;  // the exponent of a block of zeros
 
 FX_HD i64 make(u32 hi, u32 lo) { return (i64)(((u64)hi << 32) | lo); }
 FX_HD u32 hi32(i64 x) { return (u32)((u64)x >> 32); }
@@ -125,6 +132,63 @@ FX_HD int excess(u32 acc, int bits) { return 64 - bits - (int)clz32(acc); }
 // x * 2^-s, rounded (ties up), -32 < s < 32
 FX_HD i64 shift_by(i64 x, int s) { return s > 0 ? (x + (1ll << (s - 1))) >> s : (i64)((u64)x << -s); }
 
+// the same for 0 <= s < 32, without a branch
+FX_HD i64 round_shift(i64 x, u32 s) { return (x + (i64)((1u << s) >> 1)) >> s; }
+
+// the same for any s; 0 from s = 63 on
+FX_HD i64 shift_any(i64 x, int s)
+{
+    if (s <= 0) return (i64)((u64)x << (s > -63 ? -s : 63));
+    return s < 63 ? (x + (1ll << (s - 1))) >> s : 0;
+}
+
+FX_HD int bits_of_word(u64 u)  // of an unsigned number, 0 for 0
+{
+    const u32 h = (u32)(u >> 32), l = (u32)u;
+    return h ? 64 - (int)clz32(h) : 32 - (int)clz32(l);
+}
+
+// a word of as many bits as |x| has (or |x| - 1, for negative x), 0 only for 0; for several values the union
+FX_HD u64 mag64(i64 x) { return (u64)(x ^ (x >> 63)) | (u64)x >> 63; }
+
+struct Cx {
+    i64 r, i;
+};
+
+FX_HD u32 spread(Cx x) { return spread(x.r) | spread(x.i); }
+FX_HD u64 mag64(Cx x) { return mag64(x.r) | mag64(x.i); }
+// b >= 1 with |x| <= 2^b; 0 for 0
+template <class T>
+FX_HD int bits64(T x) { return bits_of_word(mag64(x)); }
+FX_HD Cx round_shift(Cx x, u32 s) { return Cx{round_shift(x.r, s), round_shift(x.i, s)}; }
+FX_HD Cx shift_any(Cx x, int s)
+{
+    if (s <= 0) return Cx{(i64)((u64)x.r << (s > -63 ? -s : 63)), (i64)((u64)x.i << (s > -63 ? -s : 63))};
+    const u32 r = s < 63 ? (u32)s : 63u;
+    const i64 half = (i64)((1ull << r) >> 1);
+    return s < 63 ? Cx{(x.r + half) >> r, (x.i + half) >> r} : Cx{0, 0};
+}
+
+// Register k's group where 16 registers hold G groups, numbered by the high or the low bits of k.
+template <int G, bool HIGH>
+FX_HD constexpr int group_of(int k) { return HIGH ? k / (16 / G) : k % G; }
+template <int G, bool HIGH>
+FX_HD constexpr int member_of(int g, int i) { return HIGH ? g * (16 / G) + i : i * G + g; }
+
+// The exponent that N values x(i) of exponents e(i) are brought to: the largest just below 2^bits, in units
+// of 2^low at least; E_ZERO where all are 0.
+template <class X, class E>
+FX_HD int common_exponent(int n, int bits, int low, X x, E e)
+{
+    int top = E_ZERO;
+    FX_UNROLL2
+    for (int i = 0; i < n; i++) {
+        const int b = bits64(x(i));
+        top = b && b + e(i) > top ? b + e(i) : top;
+    }
+    return top == E_ZERO ? E_ZERO : top - bits > low ? top - bits : low;
+}
+
 // A 64-bit integer as hi * 2^32 + lo with both halves signed.
 struct Halves {
     int hi, lo;
@@ -161,10 +225,6 @@ FX_HD i64 mul_real(i64 x, Halves w)
     m = (i64)v.lo * w.hi + m;
     return (i64)((u64)h << 2) + (m >> 30);
 }
-
-struct Cx {
-    i64 r, i;
-};
 
 // A complex factor c + i d, with t = d and s = -d: the conjugate swaps the two.
 struct Tw {
@@ -267,11 +327,57 @@ FX_HD void dft2(Cx &x0, Cx &x1)
     x1 = Cx{a.r - x1.r, a.i - x1.i};
 }
 
+// Between its two halves a group's values fall into classes that do not mix again: the values of a class
+// that the first half's adds have left small are shifted up, so that the rotations round beside
+// them and not beside the group's largest.  Lifts has the shift of each class.
+struct Lifts {
+    int s[4];
+};
+
+// What a transform does between its halves, operator()<forward>(values, shifts): nothing, for blocks alike.
+struct NoLift {
+    template <bool FWD>
+    FX_HD void operator()(Cx (&)[16], Lifts &) const
+    {
+    }
+};
+
+// Whether a class (registers k & 3 forward, k >> 2 inverse; class 0 takes no rotation) may need a lift: three
+// of its four values are looked at, of which with data whose outputs are alike in size one is large
+// enough but in one thread of a million.
+template <bool FWD>
+FX_HD bool may_lift(const Cx (&x)[16])
+{
+    bool small = false;
+    FX_UNROLL
+    for (int j = 1; j < 4; j++)
+        small = small || !((FWD ? spread(x[j]) | spread(x[j + 4]) | spread(x[j + 8])
+                                : spread(x[4 * j]) | spread(x[4 * j + 1]) | spread(x[4 * j + 2])) >> 21);
+    return small;
+}
+
+// The shift that brings four values of magnitudes `mag` to below 2^60 (rotations and two more stages fit), where
+// that is seven bits and more, `room` at most.
+FX_HD int lift_of(u64 mag, int room)
+{
+    if (mag >> 53 || !mag) return 0;
+    int s = 60 - bits_of_word(mag);
+    s = s < room ? s : room;
+    return s > 0 ? s : 0;
+}
+
+// The class of register k of a forward / inverse transform on NB bits.
+template <int NB>
+FX_HD constexpr int dft_class(int k) { return NB >= 3 ? k & 3 : 0; }
+template <int NB>
+FX_HD constexpr int idft_class(int k) { return NB >= 3 ? k >> 2 : 0; }
+
 // The stages on the upper NB bits of a 4-bit register index (the lower 4 - NB bits
 // number independent groups): forward, input bit-reversed.
-template <int NB>
-FX_HD void dft_regs(Cx (&x)[16])
+template <int NB, class L>
+FX_HD Lifts dft_regs(Cx (&x)[16], L lift)
 {
+    Lifts s{{0, 0, 0, 0}};
     if (NB == 1) {
         FX_UNROLL
         for (int k = 0; k < 8; k++) dft2(x[k], x[k + 8]);
@@ -279,6 +385,7 @@ FX_HD void dft_regs(Cx (&x)[16])
     if (NB == 4) {
         FX_UNROLL
         for (int k = 0; k < 16; k += 4) dft4(x[k], x[k + 1], x[k + 2], x[k + 3]);
+        lift.template operator()<true>(x, s);
         x[5] = rot16<2, false>(x[5]);
         x[9] = rot16<1, false>(x[9]);
         x[13] = rot16<3, false>(x[13]);
@@ -292,6 +399,7 @@ FX_HD void dft_regs(Cx (&x)[16])
             dft2(x[k], x[k + 2]);
             dft2(x[k + 1], x[k + 3]);
         }
+        lift.template operator()<true>(x, s);
         x[7] = rot16<4, false>(x[7]);
         x[11] = rot16<2, false>(x[11]);
         x[15] = rot16<6, false>(x[15]);
@@ -305,12 +413,16 @@ FX_HD void dft_regs(Cx (&x)[16])
         FX_UNROLL
         for (int g = 0; g < 4; g++) dft4(x[g], x[g + 4], x[g + 8], x[g + 12]);
     }
+    return s;
 }
+template <int NB>
+FX_HD void dft_regs(Cx (&x)[16]) { dft_regs<NB>(x, NoLift{}); }
 
 // the inverse, output bit-reversed
-template <int NB>
-FX_HD void idft_regs(Cx (&x)[16])
+template <int NB, class L>
+FX_HD Lifts idft_regs(Cx (&x)[16], L lift)
 {
+    Lifts s{{0, 0, 0, 0}};
     if (NB == 1) {
         FX_UNROLL
         for (int k = 0; k < 8; k++) dft2(x[k], x[k + 8]);
@@ -320,6 +432,7 @@ FX_HD void idft_regs(Cx (&x)[16])
         for (int g = 0; g < 4; g++) idft4(x[g], x[g + 4], x[g + 8], x[g + 12]);
     }
     if (NB >= 3) {
+        lift.template operator()<false>(x, s);
         x[6] = rot16<4, true>(x[6]);
         x[10] = rot16<2, true>(x[10]);
         x[14] = rot16<6, true>(x[14]);
@@ -344,7 +457,10 @@ FX_HD void idft_regs(Cx (&x)[16])
         FX_UNROLL
         for (int k = 0; k < 16; k += 4) idft4(x[k], x[k + 1], x[k + 2], x[k + 3]);
     }
+    return s;
 }
+template <int NB>
+FX_HD void idft_regs(Cx (&x)[16]) { idft_regs<NB>(x, NoLift{}); }
 
 // Walsh-Hadamard stages on register bits LO .. HI-1
 template <int LO, int HI>

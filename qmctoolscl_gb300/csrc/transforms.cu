@@ -24,11 +24,14 @@
 //
 // GB300 runs FP64 at about 1.25 TFLOP/s, so these FP64 stages (ft_pass_kernel) are bound by the
 // FP64 unit.  From 2^9 values on the passes of fix_transform.cuh take their place: the same
-// transform with each tile in 64-bit block fixed point on the integer and IMAD pipes (errors
-// against long double: 0.3-0.9 of the FP64 stages' on normal, spiky, smooth and nearly
-// constant data, n = 2^9..2^18).  Device time, FP64 stages -> fixed point: FFT of
-// 32 x 2^20 4500 -> 1070 us, IFFT of 111 x 2^10 17.2 -> 16.6, WHT of 300 x 2^16 845 -> 144.
-// The tensor-core path (tc_fft.cu) is faster still at 1e-7.
+// transform in 64-bit block fixed point on the integer and IMAD pipes, an exponent for every 16 values that
+// go through four stages together.  Errors against long double, n = 2^9..2^16: 0.2-0.9 of the FP64
+// stages' in L2 on normal, lognormal, smooth and nearly constant data and kernel columns, and no larger
+// output by output (median and 90th percentile of |error| / |output|).  What is left of the block: a value
+// that is 2^5 and more below another of its 16 keeps 58 bits below that one's size, which shows where the large ones
+// cancel exactly and the small ones do not.  Device time, FP64 stages -> fixed point: FFT of
+// 32 x 2^20 4490 -> 1111 us, IFFT of 111 x 2^10 17.2 -> 15.2, WHT of 300 x 2^16 843 -> 152.
+// The tensor-core path (tc_fft.cu) is faster still at 1e-7, but for the WHT.
 #include <cmath>
 
 #include "common.cuh"

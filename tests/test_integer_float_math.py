@@ -77,3 +77,15 @@ def test_block_fixed_point(fix64_checker, seed):
     out = subprocess.run([fix64_checker, "200000", str(seed)], capture_output=True, text=True, timeout=120)
     assert out.returncode == 0, out.stdout + out.stderr
     assert out.stdout.startswith("ok")
+
+
+@pytest.fixture(scope="module")
+def fix_exponents_checker(tmp_path_factory):
+    return _compile(tmp_path_factory, "fix_exponents_check.cpp")
+
+
+@pytest.mark.parametrize("seed", [1, 2])
+def test_block_exponents(fix_exponents_checker, seed):
+    out = subprocess.run([fix_exponents_checker, "200000", str(seed)], capture_output=True, text=True, timeout=120)
+    assert out.returncode == 0, out.stdout + out.stderr
+    assert out.stdout.startswith("ok")
