@@ -1662,7 +1662,7 @@ def run_gdn_nus(args):
                              "seconds": t_cpu}}
 
 
-# the default run's "configs" object: every other configuration of the benchmark, each its own
+# the default run's "configs": every other configuration of the benchmark, each its own
 # workload function (the same as --workload <name>), with at most this many timed steps
 CONFIGS = [("cfg1_net_plain", "net_plain", 10), ("cfg3_net_lms", "net_lms", 10), ("cfg4_halton", "halton", 10),
            ("cfg5_fft", "fft", 10), ("plain_drop_in", "plain", 10), ("halton_qrng", "qrng", 10),
@@ -1696,6 +1696,36 @@ def run_configs(args):
     return out
 
 
+def headline(line):
+    """(the line to print, the details for standard error): the line has to fit what a log's tail keeps, 3000 characters.
+    Of the other configurations it carries the value and the milliseconds, of the other end-to-end forms the
+    values."""
+    short, details = dict(line), {}
+    for key in ("cpu_as_shipped", "configs"):
+        if key in short:
+            details[key] = short.pop(key)
+    if "configs" in details:
+        short["configs"] = {k: {"error": v["error"][:60]} if "error" in v else
+                            {"value": v["value"], "unit": v["unit"].split()[0], "ms": v["ms_per_step"]}
+                            for k, v in details["configs"].items()}
+    if "other" in short.get("e2e", {}):
+        short["e2e"] = dict(short["e2e"])
+        details["e2e"] = {k: short["e2e"].pop(k) for k in ("other", "link") if k in short["e2e"]}
+        short["e2e"]["other"] = {k: v["value"] for k, v in details["e2e"]["other"].items()}
+    return six_digits(short), details
+
+
+def six_digits(v):
+    """Floats of a line to six significant digits."""
+    if isinstance(v, float):
+        return float("%.6g" % v)
+    if isinstance(v, dict):
+        return {k: six_digits(x) for k, x in v.items()}
+    if isinstance(v, (list, tuple)):
+        return [six_digits(x) for x in v]
+    return v
+
+
 WORKLOADS = {"net_plain": run_net_plain, "net_lms": run_net_lms, "fft": run_fft, "halton": run_halton,
              "plain": run_gdn_plain, "gdn_plain": run_gdn_plain, "qrng": run_qrng, "nus": run_nus,
              "gdn_nus": run_gdn_nus}
@@ -1727,7 +1757,9 @@ def main():
         if line is not None:  # rank 0
             if line.get("n_gpus") == 1 and not args.small and not args.no_configs:
                 line["configs"] = run_configs(args)
-            print(json.dumps(line), flush=True)
+            short, details = headline(line)
+            print(json.dumps(details), file=sys.stderr, flush=True)
+            print(json.dumps(short), flush=True)
 
 
 if __name__ == "__main__":
