@@ -1213,7 +1213,7 @@ def run_halton(args):
     fp64_inst = profiled_value("halton_rows_kernel_r32_n2p18_d100.md", "fp64_warp_inst_per_launch")
     return {"metric": METRIC, "value": pts / (ms_fused / 1e3), "unit": "points/s", "n_gpus": 1,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_fused, "higher_is_better": True,
-            "scaling": "weak", "vs_baseline": None, "dtype": "u32 digits, f64 adds (split FP64 unit / integer by the tuned share)",
+            "scaling": "weak", "vs_baseline": None, "dtype": "u32 digits, f64 sums (first 16 bits of adds on the FP64 unit, the rest in integers, same bits)",
             "data": "synthetic (np.random.SFC64(4)): reference generators per dimension",
             "config": {"workload": "randomised Halton, bases = first 100 primes, d=100, n=2^18, r=32, "
                                    "tmax_j=ceil(64/log2 b), LMS + permutation + digital shift + float "
@@ -1439,7 +1439,7 @@ def run_qrng(args):
             "roofline": dict(roofline(8.0 * n * d, ms), kernel="halton_qrng_kernel",
                              note="bound by instruction issue on two units, not by HBM: about one step a point (the "
                                   "values of the high digits are shared), the reference's rounded add and divide, half "
-                                  "of the steps on the FP64 pipe and half in integer arithmetic (ncu: FP64 pipe 71 %, "
+                                  "of the steps on the FP64 pipe and half in integer arithmetic (ncu: FP64 pipe 70 %, "
                                   "ALU 62 %; profiles/halton_qrng_kernel_n2p20_d100.md)"),
             "gpu_launches": args.steps,
             "cpu_baseline": {"value": ns / t_cpu, "unit": "points/s (d=100)", "cores": threads, "kind": "port",

@@ -11,9 +11,9 @@
 //         rows, 256 threads: two groups, or one that stays in registers.
 // Exponents: a thread's 16 values have one of their own where their size asks for it (fix64.cuh), and the tile
 // one in common where all blocks are alike, as random data's are.
-// What bounds it: the ALU pipe (55-75 % busy over the pass, IMAD 20 %, HBM 24-50 %) and the
-// barriers between the groups' phases; FFT of 32 x 2^20 in 0.55 + 0.56 ms, WHT of 300 x 2^16 in 85 +
-// 67 us.  Sixteen complex values a thread (128 registers, 2 CTAs of 8 warps per SM) hold a
+// What bounds it: latency and the integer pipes together, with 14 warps of 16 per SM resident for complex data (issue 43-47 %,
+// ALU 40-43 %, IMAD 46-56 %, stalls spread over waits, shared memory and the pipes), the ALU for real
+// data (64 %, FP64 conversions 39-60 %); FFT of 32 x 2^20 in 0.55 + 0.56 ms, WHT of 300 x 2^16 in 89 + 60 us.  Sixteen complex values a thread (128 registers, 2 CTAs of 8 warps per SM) hold a
 // radix-16 group: three exchanges for 12 bits where radix 4 in shared memory had six.
 // Lengths below 2^9 keep the FP64 pass.  A tile that holds an inf or a nan, or blocks of values near the
 // ends of the exponent range, is done by the FP64 stages.

@@ -82,7 +82,7 @@ __global__ void nus_keys_kernel(NusDims m, const u64 *__restrict__ xb, const u64
 // come first (one warp per 256 points, then a scan per generator); the stream itself, the only
 // serial part, then runs without looking at the draws; and the draws take their bits from it, a
 // thread per point.  With the draws formatted and stored inside the serial loop, a step took
-// 68 cycles; the bare chain of 64-bit integer operations takes 24 on one warp (32
+// 68 cycles; the bare chain of 64-bit integer operations takes 24 on one warp (up to 32
 // generators: the ALU).  r=4, d=8, n=200000: 7.15 ms for the draws before, 2.59 now (stream 2.53).
 
 constexpr u32 DT = 256;  // points per warp of the counting and formatting passes: all loads in flight at once

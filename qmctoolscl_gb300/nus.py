@@ -19,8 +19,9 @@ computes in parallel instead of walking the tree:
 
 The kernels sort each generator's keys, build a binary radix tree over them,
 take each subtree's earliest point bottom-up (which gives every L_v), run the
-draws (one thread per generator, numpy's SFC64 stream and bounded-integer
-rule), and OR each point's bits from its ancestors' draws.
+generators' streams (a lane each, numpy's SFC64) for as many outputs as the draws
+take, format the draws from them (a thread each, numpy's bounded-integer rule),
+and OR each point's bits from its ancestors' draws.
 
 Generators must be ``numpy.random.Generator(numpy.random.SFC64(...))`` (the
 reference's own family), one per (l, j) pair, as the reference's documented

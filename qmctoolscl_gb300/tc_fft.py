@@ -4,7 +4,10 @@ Walsh-Hadamard transform with radix-16 steps as BF16 tensor-core products
 functions minus the twiddle arrays: fft_bro_1d_tc(d1, d2, n_half, xr, xi),
 ifft_bro_1d_tc(d1, d2, n_half, xr, xi), fwht_1d_tc(d1, d2, n_half, x), in
 place on numpy arrays (copied to the GPU and back) or CUDA float64 tensors.
-Relative L2 error about 1e-7 against the FP64 transforms.
+Relative L2 error about 1e-7 against the FP64 transforms.  4096 vectors of
+2^10..2^20: FFT 14.1 ms against 24.8 of the FP64 call; the Walsh-Hadamard form is
+slower than the FP64 call (fwht_1d_radix2: 6.2 ms, fwht_1d_tc: 8.1) and far less
+exact, and kept for callers that have it.
 
 fft_mul_ifft_tc(d1, d2, n_half, lam_r, lam_i, xr, xi, divide=False, scale=1.0)
 is the fast kernel matrix-vector product (divide=False: ifft(fft(y) * lam) *
