@@ -581,7 +581,7 @@ __global__ void __launch_bounds__(1 << (P - 4), P == 12 ? 2 : (P == 11 ? 4 : (P 
     const Places<Cx> top{sr, si, slot(t), T + T / 16};
     const Places<Cx> mid{sr, si, (t & 15u) + 272u * (t >> 4), 17};
     const Places<Cx> low{sr, si, 17u * t, 1};
-    const int lowest = low_exponent(a);
+    const int lowest = low_exponent(a), lowest1 = KIND == FT_CONV ? -1022 : lowest;  // lowest1: of a fused pass's first half
     const u64 tiles = a.nvec << (a.m - P);
     for (u64 tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const u64 base = tile << P;
@@ -607,22 +607,22 @@ __global__ void __launch_bounds__(1 << (P - 4), P == 12 ? 2 : (P == 11 ? 4 : (P 
 #pragma unroll
             for (int k = 0; k < 16; k++) x[k] = low.get(k);
             enter<fx::TOP, 1, false>(x, e, st, low, eo + t, get_max(ws[0]), some_mag(x), 0);
-            fx::Lifts s = fx::dft_regs<4>(x, LiftOwn{st, low, eo + t, e[0] - lowest});
+            fx::Lifts s = fx::dft_regs<4>(x, LiftOwn{st, low, eo + t, e[0] - lowest1});
             const int e1[4] = {e[0], e[0] - s.s[1], e[0] - s.s[2], e[0] - s.s[3]};
-            if (!redeal<fx::TOP_TW, 1, false>(x, e, e1, st, ws[1], ROW, ex[0].v[0], eo + t, lowest, low, mid,
+            if (!redeal<fx::TOP_TW, 1, false>(x, e, e1, st, ws[1], ROW, ex[0].v[0], eo + t, lowest1, low, mid,
                                               [=](int k) { return (t & 3u) * ROW + (t & ~15u) + k; })) {
                 fp64_tile<KIND>(a, sm, base, 0, 0, 1, TILE);
                 continue;
             }
             {
                 twiddle_mid<false>(x, t & 15u);
-                s = fx::dft_regs<4>(x, LiftOwn{st, mid, eo + t, e[0] + 2 - lowest});
+                s = fx::dft_regs<4>(x, LiftOwn{st, mid, eo + t, e[0] + 2 - lowest1});
                 const int e2[4] = {e[0] + 2, e[0] + 2 - s.s[1], e[0] + 2 - s.s[2], e[0] + 2 - s.s[3]};
-                redeal<fx::TOP_TW, G, false>(x, et, e2, st, ws[2], ROW, ex[1].v[0], eo + t, lowest, mid, top, [=](int k) {
+                redeal<fx::TOP_TW, G, false>(x, et, e2, st, ws[2], ROW, ex[1].v[0], eo + t, lowest1, mid, top, [=](int k) {
                     return (((t >> 4) | (k * T / 16 & 15u)) & 3u) * ROW + ((k * T >> 8) << 4 | (t & 15u));
                 });
                 twiddle_top<P>(x, t);
-                s = fx::dft_regs<NB>(x, LiftOwn{st, top, eo + t, room(et, lowest)});
+                s = fx::dft_regs<NB>(x, LiftOwn{st, top, eo + t, room(et, lowest1)});
 #pragma unroll
                 for (int k = 0; k < 16; k++) own[k] = et[fx::group_of<G, false>(k)] + 2 - s.s[fx::dft_class<NB>(k)];
             }
@@ -696,7 +696,7 @@ __global__ void __launch_bounds__(256, 2) fix_high_kernel(PassArgs a)
     const u32 t = threadIdx.x;
     const Places<Cx> top{sr, si, slot(t), 272};
     const Places<Cx> mid{sr, si, (t & 15u) + 272u * (t >> 4), 17};
-    const int lowest = low_exponent(a);
+    const int lowest = low_exponent(a), lowest1 = KIND == FT_CONV ? -1022 : lowest;  // lowest1: of a fused pass's first half
     const u64 chunks = (1ull << a.k0) / CT;
     const u64 tiles = (a.nvec << (a.m - a.k1)) * chunks;
     const u32 col = S == 8 ? (t & 15u) : t, q = S == 8 ? t >> 4 : 0u;
@@ -742,17 +742,17 @@ __global__ void __launch_bounds__(256, 2) fix_high_kernel(PassArgs a)
                 twiddle_columns<false>(x, wa, tba, tbb, col);
             else
                 twiddle_powers<CONJ, false>(x, a, c, sh);
-            fx::Lifts s = fx::dft_regs<4>(x, LiftOwn{st, S == 8 ? mid : top, eo + t, e[0] + 2 - lowest});
+            fx::Lifts s = fx::dft_regs<4>(x, LiftOwn{st, S == 8 ? mid : top, eo + t, e[0] + 2 - lowest1});
             if (S == 8) {
                 const int e1[4] = {e[0] + 2, e[0] + 2 - s.s[1], e[0] + 2 - s.s[2], e[0] + 2 - s.s[3]};
-                if (!redeal<fx::TOP_TW, 1, false>(x, e, e1, st, ws[1], ROW, ex[0].v[0], eo + t, lowest, mid, top,
+                if (!redeal<fx::TOP_TW, 1, false>(x, e, e1, st, ws[1], ROW, ex[0].v[0], eo + t, lowest1, mid, top,
                                                   [=](int k) { return (q & 3u) * ROW + (k << 4 | (t & 15u)); })) {
                 fp64_tile<KIND>(a, sm, base, tile / chunks, c0, CT, 4096);
                 continue;
             }
                 {
                     twiddle_mid<false>(x, q);
-                    s = fx::dft_regs<4>(x, LiftOwn{st, top, eo + t, e[0] + 2 - lowest});
+                    s = fx::dft_regs<4>(x, LiftOwn{st, top, eo + t, e[0] + 2 - lowest1});
                 }
             }
 #pragma unroll
@@ -833,7 +833,7 @@ __global__ void __launch_bounds__(1 << (P - 4), P == 12 ? 4 : (P == 11 ? 8 : (P 
     const Places<i64> top{sr, slot(t), T + T / 16};
     const Places<i64> mid{sr, (t & 15u) + 272u * (t >> 4), 17};
     const Places<i64> low{sr, 17u * t, 1};
-    const int lowest = low_exponent(a);
+    const int lowest = low_exponent(a), lowest1 = KIND == FT_WCONV ? -1022 : lowest;  // lowest1: of a fused pass's first half
     const u32 out = (t & 15u) + ((t >> 4) << 8);  // the middle deal's place in the tile, + 16 k
     const u64 tiles = a.nvec << (a.m - P);
     for (u64 tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
@@ -850,14 +850,14 @@ __global__ void __launch_bounds__(1 << (P - 4), P == 12 ? 4 : (P == 11 ? 8 : (P 
         int e[1], eg[G], own[16];
         enter<fx::TOP, 1, false>(x, e, st, top, eo + t, get_max(ws[0]), mx, 0);
         fx::wht_regs<0, 4>(x);
-        if (!redeal<fx::TOP, 1, false>(x, e, e, st, ws[1], ROW, ex[0].v[0], eo + t, lowest, top, low,
+        if (!redeal<fx::TOP, 1, false>(x, e, e, st, ws[1], ROW, ex[0].v[0], eo + t, lowest1, top, low,
                                        [=](int k) { return (16 * t + k) & (T - 1); })) {
                 fp64_tile<KIND>(a, sm, base, 0, 0, 1, TILE);
                 continue;
             }
         {
             fx::wht_regs<0, 4>(x);
-            redeal<fx::TOP, G, true>(x, eg, e, st, ws[2], ROW, ex[1].v[0], eo + t, lowest, low, mid,
+            redeal<fx::TOP, G, true>(x, eg, e, st, ws[2], ROW, ex[1].v[0], eo + t, lowest1, low, mid,
                                      [=](int k) { return (t & ~15u) + k; });
             fx::wht_regs<0, P - 8>(x);
 #pragma unroll
@@ -908,7 +908,7 @@ __global__ void __launch_bounds__(256, 4) fix_high_wht_kernel(PassArgs a)
     const u32 t = threadIdx.x;
     const Places<i64> top{sr, slot(t), 272};
     const Places<i64> mid{sr, (t & 15u) + 272u * (t >> 4), 17};
-    const int lowest = low_exponent(a);
+    const int lowest = low_exponent(a), lowest1 = KIND == FT_WCONV ? -1022 : lowest;  // lowest1: of a fused pass's first half
     const u64 chunks = (1ull << a.k0) / CT;
     const u64 tiles = (a.nvec << (a.m - a.k1)) * chunks;
     const u32 col = S == 8 ? (t & 15u) : t, q = S == 8 ? t >> 4 : 0u;
@@ -937,7 +937,7 @@ __global__ void __launch_bounds__(256, 4) fix_high_wht_kernel(PassArgs a)
             enter_alone<fx::TOP>(x, e, st, mid, eo + t, 0);
         fx::wht_regs<0, 4>(x);
         if (S == 8) {
-            if (!redeal<fx::TOP, 1, false>(x, e, e, st, ws[1], ROW, ex[0].v[0], eo + t, lowest, mid, top,
+            if (!redeal<fx::TOP, 1, false>(x, e, e, st, ws[1], ROW, ex[0].v[0], eo + t, lowest1, mid, top,
                                            [=](int k) { return k << 4 | (t & 15u); })) {
                 fp64_tile<KIND>(a, sm, base, tile / chunks, c0, CT, 4096);
                 continue;

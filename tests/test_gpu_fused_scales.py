@@ -38,3 +38,22 @@ def test_scales(m, nv, divide, log2_scale, magnitude, log2_lam):
         err = np.sqrt((((y - want) / top) ** 2).sum(axis=1)) / np.sqrt(((want / top) ** 2).sum(axis=1))
         assert (np.abs(y - want) <= low).all() or err.max() < 2e-15, err.max()
     assert np.abs(xi).max() <= max(low, 1e-13 * float(top))
+
+
+@pytest.mark.parametrize("m,nv", [(9, 200), (10, 2), (12, 2), (13, 2), (17, 1), (20, 1)])
+@pytest.mark.parametrize("log2_scale,log2_data,log2_lam", [(-600, -400, 300), (600, 300, -500), (-200, -700, 500), (0, -700, 0)])
+def test_scales_with_blocks_apart(m, nv, log2_scale, log2_data, log2_lam):
+    """A constant with a little noise, whose blocks take exponents of their own, small and with a scale far from 1."""
+    rng = np.random.Generator(np.random.SFC64(m))
+    n = 1 << m
+    z = np.ldexp(1 + 1e-9 * rng.standard_normal((nv, n)), log2_data)
+    scale, lam = 2.0 ** log2_scale, np.full(n, 2.0 ** log2_lam)
+    x, xr, xi = z.copy(), z.copy(), np.zeros_like(z)
+    tc_fft.fwht_mul_fwht(nv, 1, n // 2, lam, x, scale=scale)
+    tc_fft.fft_mul_ifft(nv, 1, n // 2, lam, np.zeros(n), xr, xi, scale=scale)
+    back = -(log2_scale + log2_lam)
+    for y in (x, xr):
+        # halves of the way back: the whole factor need not be a double
+        y = np.ldexp(np.ldexp(y, back // 2 - log2_data // 2), back - back // 2 - (log2_data - log2_data // 2))
+        one = np.ldexp(z, -log2_data)
+        assert np.abs(y - one).max() < 4e-15
