@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(FT_THREADS) ft_pass_kernel(PassArgs a)
     }
 }
 
-// One tile of a fixed-point pass in FP64 (tiles that hold inf, nan, zeros only or values near the
+// One tile of a fixed-point pass in FP64 (tiles that hold inf, nan or a block of values near the
 // ends of the exponent range): starts from and ends with the data in global memory, and with
 // a barrier.
 template <int KIND>
@@ -422,11 +422,12 @@ int launch_pass(int kind, bool conj, const PassArgs &a, unsigned grid, size_t sm
 // ---- the fixed-point passes
 
 // Few complex transforms of 2^9 are latency-bound, and the FP64 stages on 256 threads each
-// answer sooner than one warp does (64 vectors: 12.7 us against
-// 14.4; 300: 16.6 against 14.4; from 2^10 on fixed point wins from one vector: 15.6 against 17.9).
+// answer sooner than one warp does, up to a vector per SM (FFT of 152 vectors: 12.6 us against
+// 15.3; 200: 16.6 against 15.8; from 2^10 on fixed point wins from one vector, 15.0 against 17.4, but for
+// data whose blocks take exponents of their own: 24, and from 2^11 on, 26 against 31).
 bool use_fixed(bool real, u32 m, u64 nvec)
 {
-    return m > (u32)FIX_MIN_BITS || (m == (u32)FIX_MIN_BITS && (real || nvec >= (u64)qmcgb::sm_count()));
+    return m > (u32)FIX_MIN_BITS || (m == (u32)FIX_MIN_BITS && (real || nvec > (u64)qmcgb::sm_count()));
 }
 
 // Bits of the low pass of an m-bit transform: what is left above it is a multiple of four.
