@@ -158,7 +158,7 @@ inline unsigned grid_for(u64 work, unsigned per_block, unsigned cap)
 int sm_count();
 
 // Raise the kernel's dynamic shared-memory limit to at least `bytes` (no-op up
-// to the default 48 KB).  The limit is one attribute per kernel and device:
+// to the default: 48 KB less the kernel's static arrays).  The limit is one attribute per kernel and device:
 // it is only ever raised (a high-water mark kept under a lock), so a launch
 // prepared for one size is never broken by a later, smaller setting.
 int raise_smem_limit(const void *func, size_t bytes, const char *what);

@@ -32,13 +32,19 @@ int launch_status(const char *what) { return cuda_status(cudaGetLastError(), wha
 
 int raise_smem_limit(const void *func, size_t bytes, const char *what)
 {
-    if (bytes <= 48 * 1024) return QMC_OK;
     static std::mutex mu;
     static std::map<std::pair<int, const void *>, size_t> high;
     int dev = 0;
     if (int rc = cuda_status(cudaGetDevice(&dev), what)) return rc;
     std::lock_guard<std::mutex> lock(mu);
-    size_t &cur = high[{dev, func}];
+    auto found = high.find({dev, func});
+    if (found == high.end()) {  // without an attribute 48 KB, the kernel's static arrays included
+        cudaFuncAttributes at{};
+        if (int rc = cuda_status(cudaFuncGetAttributes(&at, func), what)) return rc;
+        const size_t most = 48 * 1024;
+        found = high.insert({{dev, func}, at.sharedSizeBytes < most ? most - at.sharedSizeBytes : 0}).first;
+    }
+    size_t &cur = found->second;
     if (bytes <= cur) return QMC_OK;
     if (int rc = cuda_status(cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes), what))
         return rc;

@@ -36,6 +36,24 @@ def test_rule(r, n, bases, tables):
     assert plan.info() == {"has_tables": tables, "uses_tables": tables}
 
 
+@pytest.mark.parametrize("b", [2, 3, 4, 5, 8, 16, 25, 31, 32, 37, 64, 101, 128, 211, 256, 509])
+def test_one_dimension(b):
+    """Plans of one dimension, small tables: some of them fit the 48 KB that a kernel has unasked only without the
+    kernel's static arrays."""
+    import torch
+    plan, _, x = _plan(1, 2400007, [b])
+    assert plan.info()["uses_tables"]
+    plan.prepare()
+    plan.run()
+    torch.cuda.synchronize()
+    got = x.clone()
+    plan.set_fp64_share(0.5)
+    x.fill_(-1.0)
+    plan.run()
+    torch.cuda.synchronize()
+    assert torch.equal(x.view(torch.int64), got.view(torch.int64))
+
+
 def test_pinned_output_has_no_tables():
     from qmctoolscl_gb300 import batch
     plan, _, _ = _plan(2, 130001, PRIMES[:12], batch.pinned_empty((2, 130001, 12)))
