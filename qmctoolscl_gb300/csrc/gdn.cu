@@ -768,6 +768,7 @@ struct I2fDim {
     u32 b, t1, tr, off;
 };
 
+constexpr u32 I2F_TABLE_VALUES = 500;
 constexpr u32 I2F_CTAS = 2;               // per SM (3 with 8 digits at a time: 244 us for 229)
 constexpr u32 I2F_CHUNK = 16;             // digits of a point copied at a time: a line
 constexpr u32 I2F_ROW = I2F_CHUNK * 8 + 16;  // and its place in a warp's buffer (padded: no bank conflicts)
@@ -893,9 +894,8 @@ __device__ bool i2f_tables(const u64 *bl, u32 nd, u64 tmax, I2fDim *dims)
 // another, 16 digits at a time, the next 16 on their way to shared memory; the products come from the
 // tables and the sum from integers after the first rows.  d=4, bases 2, 3, 5, 7, tmax=32, 2^20 points:
 // 358 us with an FP64 add per digit (the unit 83 % busy) and each lane reading its own point, 229
-// now (ALU 35 %, FP64 31 %: 16 warps per SM wait for one another's phases).  One wave of CTAs: the tables (a serial
-// chain of divides) cost as much as 500 points.  Below 16 digits a unit is too short to hide its
-// copies (base 541, 8 digits: 163 us without, 202 with).
+// now (ALU 35 %, FP64 31 %: 16 warps per SM wait for one another's phases).  A CTA's tables (a serial
+// chain of divides) cost as much as I2F_TABLE_VALUES values: few CTAs (i2f_staged_splits).
 __global__ void __launch_bounds__(THREADS, I2F_CTAS)
     gdn_terms_float_kernel(u64 r, u64 n, u64 d, u64 r_b, u64 tmax, const u64 *bases, const u64 *xdig, double *x,
                            u64 rows_per_cta, u32 dim_tiles, u64 l_off)
@@ -1144,6 +1144,29 @@ PointGrid point_grid(u64 r, u64 n, u64 d, u64 per_point, u32 dim_tile, u64 *spli
     return pg;
 }
 
+// CTAs per randomisation and dimension tile of gdn_terms_float_kernel; 0: gdn_to_float_kernel does better.  The
+// least that fills a wave, or a number whose waves are a tenth shorter, a wave taking a CTA's values and its
+// tables (64 randomisations of 2^12 points in 16 dimensions: 177 us by 4 CTAs each, 201 by 14); and the kernel only
+// where those waves carry two values for each three that fit them: one randomisation of 2^18 values in 32 digits 33.1 us by
+// this kernel and 32.2 by the other, 2^19 values 46.5 and 67.9; 512 randomisations of 2^8 values 35.9 and 22.8.
+// Not below 16 digits, where a unit is too short to hide its copies (base 541, 8 digits: 163 us without, 202
+// with), and not with 17, 18, 19 and 21, whose second unit copies one to three digits of a point, or five by 8
+// bytes (4M values: 17 digits 1.19 times the other's time, 18 1.04, 19 1.11, 21 1.07, but 16 0.86, 20 0.98, 22 0.92).
+u64 i2f_staged_splits(u64 r, u64 n, u64 d, u64 tmax)
+{
+    const u64 nd = d < I2F_DIMS ? d : I2F_DIMS, tiles = (d + I2F_DIMS - 1) / I2F_DIMS;
+    if (tmax < I2F_STAGED || tmax > I2F_TMAX || (tmax > 16 && tmax < 20) || tmax == 21) return 0;
+    if (tmax * 2 * nd > I2F_SMEM_WORDS) return 0;  // the smallest tables: base 2 in every dimension
+    const u64 slots = (u64)qmcgb::sm_count() * I2F_CTAS, ctas = r * tiles;
+    const u64 least = ctas < slots ? slots / ctas : 1;
+    u64 best = 0, time = ~0ull;
+    for (u64 k = least; k <= least + 16 && k <= n; k++) {
+        const u64 t = (k * ctas + slots - 1) / slots * ((n + k - 1) / k * nd + I2F_TABLE_VALUES);
+        if (k == least || t * 10 < time * 9) best = k, time = t;
+    }
+    return r * n * d / slots * 3 >= time * 2 ? best : 0;
+}
+
 // launch over blockIdx.y = (randomisation, dimension tile) in chunks of 65535
 template <typename F>
 int launch_points(u64 r, u32 dim_tiles, F &&launch_chunk, const char *what)
@@ -1291,14 +1314,12 @@ int qmc_gdn_integer_to_float(uint64_t r, uint64_t n, uint64_t d, uint64_t r_b, u
     if (r == 0 || n == 0 || d == 0) return QMC_OK;
     QMC_REQUIRE(r_b > 0 && bases && x && (tmax == 0 || xdig), "bad r_b or null array pointer");
     u64 splits;
-    // the smallest tables: base 2 in every dimension
-    const bool staged = tmax >= I2F_STAGED && tmax <= I2F_TMAX && tmax * 2 * (d < I2F_DIMS ? d : I2F_DIMS) <= I2F_SMEM_WORDS;
-    if (staged) {
+    const u64 staged_splits = i2f_staged_splits(r, n, d, tmax);
+    if (staged_splits) {
         const size_t smem = (I2F_SMEM_WORDS + i2f_recip_words(d, tmax)) * sizeof(double) + THREADS / 32 * 2 * I2F_BUF;
         if (int rc = qmcgb::raise_smem_limit((const void *)gdn_terms_float_kernel, smem, "gdn_integer_to_float")) return rc;
         PointGrid pg = point_grid(r, n, d, 1, I2F_DIMS, &splits, I2F_CTAS);
-        // one wave: a split less where the rounding up made it more
-        if (splits > 1 && splits * r * pg.dim_tiles > (u64)qmcgb::sm_count() * I2F_CTAS) splits--;
+        splits = staged_splits;
         pg.rows_per_cta = (n + splits - 1) / splits;
         if (int rc = launch_points(r, pg.dim_tiles, [&](u64 l0, unsigned cnt) {
                 gdn_terms_float_kernel<<<dim3((unsigned)splits, cnt, 1), THREADS, smem, QMC_STREAM(s)>>>(
@@ -1311,7 +1332,7 @@ int qmc_gdn_integer_to_float(uint64_t r, uint64_t n, uint64_t d, uint64_t r_b, u
         gdn_to_float_kernel<<<dim3((unsigned)splits, cnt, 1), THREADS, I2F_SMEM_WORDS * sizeof(double),
                               QMC_STREAM(s)>>>(
             r, n, d, r_b, tmax, (const u64 *)bases, (const u64 *)xdig, x, pg.rows_per_cta, pg.dim_tiles, l0,
-            staged ? 1u : 0u);
+            staged_splits ? 1u : 0u);
     }, "gdn_integer_to_float");
 }
 
