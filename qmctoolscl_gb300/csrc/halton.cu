@@ -279,9 +279,15 @@ __global__ void halton_tail_kernel(HPlanDev P, u32 *tail)
         const HDim &D = P.dims[R.dim0 + j];
         u32 *tl = tail + R.t_base + l * R.s_per_l + D.s_off;
         u32 m = 0;
-        for (u32 t = D.tpad; t-- > 0;) {
-            m = max(m, tl[t]);
-            tl[t] = m;
+        for (u32 t = D.tpad; t > 0; t -= min(t, 16u)) {
+            u32 v[16];  // read together: a row after another is a chain of L2 round trips
+#pragma unroll
+            for (u32 u = 0; u < 16; u++) v[u] = u < t ? tl[t - 1 - u] : 0;
+#pragma unroll
+            for (u32 u = 0; u < 16; u++) {
+                m = max(m, v[u]);
+                if (u < t) tl[t - 1 - u] = m;
+            }
         }
     }
 }
